@@ -227,6 +227,25 @@ def test_cholesky_solver_block_sizes(ctx, shape):
     assert rel(x.numpy(), xr) <= 1e-12
 
 
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 191, 257, 385, 578])
+@pytest.mark.parametrize("spread", [0, 40])
+def test_cholesky_split_products(ctx, n, spread):
+    """The factorisation's split tensor-core products at the edges of their tiles (64, 128), of the block (64) and
+    of the in-tile scan (K = 256), on a full SPD matrix M M' / n + I, its rows and columns scaled by powers of
+    two up to 2^spread.  The scaled solution is the unscaled one exactly, and the condition number is
+    about 5, so n eps cond bounds its error: 578 * 2.2e-16 * 5 = 6.4e-13."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(n)
+    M = rng.standard_normal((n, n))
+    B = M @ M.T / n + np.eye(n)
+    y = rng.standard_normal(n)
+    d = 2.0 ** rng.integers(-spread, spread + 1, n)
+    A = P.CSR.from_scipy(sp.csr_matrix(B * d[:, None] * d[None, :]))
+    x = U.Vector(ctx, n=n)
+    U.CholeskySolver(ctx).solve(U.SparseMatrix(ctx, A), U.Vector(ctx, d * (B @ y)), x)
+    assert rel(d * x.numpy(), y) <= 1e-12
+
+
 def test_cholesky_solver_factored_inverse_above_4096(ctx):
     """Coarse sizes above 4096 keep the inverse factored (Y = L^-1 and Y^T in one buffer, two
     triangular GEMVs per solve): FP64 and FP32 vectors against a direct solve."""

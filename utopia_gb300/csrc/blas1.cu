@@ -32,6 +32,11 @@ void Context::check_kernel_flags() {
     int h[4] = {0, 0, 0, 0};
     UGPU_CUDA(cudaMemcpyAsync(h, kflags.ptr, sizeof(h), cudaMemcpyDeviceToHost, stream));
     UGPU_CUDA(cudaStreamSynchronize(stream));
+    if (h[1]) {
+        UGPU_CUDA(cudaMemsetAsync(kflags.ptr, 0, kflags.bytes, stream));
+        throw Error(UGPU_ERR_CUDA, "a dense product timed out waiting for its tensor-core operations; "
+                                   "its output is invalid");
+    }
     if (h[0]) {
         UGPU_CUDA(cudaMemsetAsync(kflags.ptr, 0, kflags.bytes, stream));
         throw Error(UGPU_ERR_CUDA, "a staged SpMV kernel timed out waiting for its shared-memory copies; "

@@ -115,7 +115,8 @@ struct Context {
     Buffer partials;   // kMaxDots * kRedBlocks doubles
     Buffer scalars;    // generic device scalars (results of reductions), 256 doubles
     Buffer counters;   // last-CTA tickets of the reductions
-    Buffer kflags;     // int[4] device error flags; [0]: a staged SpMV gave up waiting for its copies
+    Buffer kflags;     // int[4] device error flags; [0]: a staged SpMV gave up waiting for its copies; [1]: a
+                       // dense product gave up waiting for its MMAs
     long long staged_test_spin = 0;  // > 0 only inside ugpu_test_staged_wait_timeout
     double *host_scalars = nullptr;  // pinned mirror
     int64_t launches = 0;            // kernels launched through this context (instrumentation)
@@ -340,7 +341,7 @@ constexpr int64_t kDenseTriMin = 4096;  // coarse sizes above which the inverse 
 struct DenseCholesky {
     Context *ctx = nullptr;
     int64_t n = 0;
-    Buffer L;      // n*n FP64, row-major, lower triangle
+    Buffer L;      // n*n FP64, row-major: the factorisation's workspace
     Buffer Ainv;   // n*n FP64 explicit inverse (L^-T L^-1), applied as one GEMV per coarse solve; for n
                    // above kDenseTriMin instead Y = L^-1 in the lower triangle and Y^T in the upper one
                    // (tri), applied as two triangular GEMVs: the same FMAs per solve without the n^3
