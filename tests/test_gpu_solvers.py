@@ -66,6 +66,26 @@ def test_cg_unpreconditioned(ctx, oracle):
     assert rel(x.numpy(), xo) <= 1e-8
 
 
+@pytest.mark.parametrize("shape", [(1, 1), (3, 1), (8, 8), (13, 5), (61, 101), (96, 64), (83, 75), (499, 156),
+                                   (312, 499), (557, 559), (560, 560), "graph4001", "graph60001"])
+@pytest.mark.parametrize("precond", ["invdiag", "none"])
+def test_cg_resident_forms(ctx, oracle, shape, precond):
+    """Small systems run as one kernel: one cluster (up to 6144 rows), one, two and four rows per thread over all
+    SMs (up to 77,824, 155,648 and 311,296 rows), and separate kernels beyond; random graphs have rows longer than
+    the eight entries kept in registers.  From a random start, 40 iterations against the oracle: the same
+    count, and an error of the order of eps times the iterations' growth, far below 1e-11."""
+    A = P.laplacian_2d(*shape) if isinstance(shape, tuple) else P.random_spd_graph(int(shape[5:]), 4, 1)
+    rng = np.random.default_rng(A.nrows)
+    b, x0 = rng.uniform(-1.0, 1.0, A.nrows), rng.standard_normal(A.nrows)
+    atol = 1e-12 * np.linalg.norm(b)
+    xo, so = oracle.cg_solve(oracle.Matrix(A), b, x0=x0, precond=precond, atol=atol, max_it=40)
+    s = cg(ctx, U.InvDiagPreconditioner(ctx) if precond == "invdiag" else None, atol=atol, max_it=40)
+    x = U.Vector(ctx, x0)
+    s.solve(U.SparseMatrix(ctx, A), U.Vector(ctx, b), x)
+    assert abs(s.solution_status()["iterates"] - so["iterates"]) <= (0 if A.nrows > 1000 else 1)
+    assert rel(x.numpy(), xo) <= 1e-11
+
+
 def test_cg_max_it_and_initial_guess(ctx, oracle):
     A, b = P.poisson2d_cg(32, 1)
     x0 = np.random.default_rng(3).standard_normal(A.nrows)

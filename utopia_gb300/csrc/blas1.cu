@@ -37,6 +37,10 @@ void Context::check_kernel_flags() {
         throw Error(UGPU_ERR_CUDA, "a dense product timed out waiting for its tensor-core operations; "
                                    "its output is invalid");
     }
+    if (h[2]) {
+        UGPU_CUDA(cudaMemsetAsync(kflags.ptr, 0, kflags.bytes, stream));
+        throw Error(UGPU_ERR_CUDA, "a resident solver kernel timed out waiting for its other CTAs; its output is invalid");
+    }
     if (h[0]) {
         UGPU_CUDA(cudaMemsetAsync(kflags.ptr, 0, kflags.bytes, stream));
         throw Error(UGPU_ERR_CUDA, "a staged SpMV kernel timed out waiting for its shared-memory copies; "

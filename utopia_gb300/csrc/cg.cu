@@ -24,31 +24,17 @@
 // (z,r) [and (z,Ap)] as it writes z, and K3 shrinks to one thread that closes the iteration: z
 // is not read back.  Off by default: measured at 192^3 (mixed form), the BF16 sweep with the two
 // FP64 dots took 96 us against 42 us without them, more than the separate K3 (48 us) it replaces.
+// Small systems without a multigrid preconditioner run the same loop in one kernel (cg_resident.cu).
 // (K0 is not folded into the SpMV: gathering z and p per nonzero doubles the FP64 FMAs of
 // the product, and FP64 FMA throughput, not HBM, then bounds it on GB300.)
 #include <cmath>
 
 #include "abi_util.cuh"
+#include "cg.cuh"
 #include "device_util.cuh"
 #include "solver.cuh"
 
 namespace ugpu {
-
-struct CgDev {
-    double rz;      // (r, z) of the current iterate
-    double pAp;     // (p, Ap)
-    double pr;      // (p, r)            (flexible form)
-    double beta;
-    double rnorm;
-    double alpha;
-    double gnorm;   // ||r|| at the stop
-    long long it;   // the reference's `it`
-    long long iterates;
-    int done;
-    int reason;
-    int converged;
-    int pad;
-};
 
 namespace {
 
@@ -410,6 +396,18 @@ public:
         if (mode != mode_ || flexible != flexible_) loop_.reset();
         mode_ = mode;
         flexible_ = flexible;
+        // Small systems: the whole solve as one resident kernel, with and without use_graphs.  The line is where
+        // separate kernels become the faster form (cg_resident.cu has the times on both sides).
+        if (mode_ != CG_GENERIC && !flexible_ && CgResident::fits(*ctx, *op)) {
+            if (!sums_.ptr) sums_.alloc(CgResident::sum_bytes(*ctx));
+            const double *dinv = mode_ == CG_JACOBI ? static_cast<InvDiag *>(pc_)->d.as<double>() : nullptr;
+            CgResident::run(*ctx, *op, b.as<double>(), x.as<double>(), dinv, z_.as<double>(), p_.as<double>(),
+                            Ap_.as<double>(), sums_.ptr, dev_.as<CgDev>(), get("atol"), (long long)get("max_it"));
+            UGPU_CUDA(cudaMemcpyAsync(host_dev_, dev_.ptr, sizeof(CgDev), cudaMemcpyDeviceToHost, ctx->stream));
+            ctx->check_kernel_flags();
+            finish(t0, l0, false, 0);
+            return;
+        }
         // r = b - A x
         {
             SpmvArgs a;
@@ -483,7 +481,7 @@ private:
     Solver *pc_ = nullptr;
     int mode_ = -1;
     bool flexible_ = false;
-    Buffer r_, z_, p_, Ap_, r32_, z32_, dev_, part_, cnt_;
+    Buffer r_, z_, p_, Ap_, r32_, z32_, dev_, part_, cnt_, sums_;
     CgDev *host_dev_ = nullptr;
     DeviceLoop loop_;
     const void *graph_x_ = nullptr;
