@@ -38,6 +38,34 @@ def test_mprgp_matches_oracle(ctx, oracle, N, scaled):
     assert abs(st["iterates"] - so["iterates"]) <= max(2, 0.05 * so["iterates"])
 
 
+@pytest.mark.parametrize("shape", [(1, 1), (5, 3), (13, 5), (96, 64), (61, 101), (499, 156), (312, 250), (640, 256),
+                                   (557, 559), (560, 560), "graph4001", "graph60001"])
+def test_mprgp_resident_forms(ctx, oracle, shape):
+    """Small problems run as one kernel: one cluster (up to 6144 rows), one, two and four rows per thread over all
+    SMs, separate kernels beyond 311,296 rows; random graphs have rows longer than the eight entries kept in
+    registers.  Twenty-five iterations with both bounds active (CG, expansion and proportioning steps) against the
+    oracle: eps times a growth of a few per iteration stays far below 1e-10."""
+    if isinstance(shape, tuple):
+        A = P.laplacian_2d(*shape)
+    else:
+        A = P.random_spd_graph(int(shape[5:]), 4, 1)
+    rng = np.random.default_rng(A.nrows)
+    b = rng.uniform(-1.0, 1.0, A.nrows)
+    lb, ub = rng.uniform(-0.3, 0.0, A.nrows), rng.uniform(0.0, 0.3, A.nrows)
+    xo, so = oracle.mprgp_solve(oracle.Matrix(A), b, lb, ub, atol=1e-12, rtol=1e-30, max_it=25)
+    s = U.MPRGP(ctx, atol=1e-12, rtol=1e-30, max_it=25)
+    vlb, vub = U.Vector(ctx, lb), U.Vector(ctx, ub)
+    s.set_box_constraints(vlb, vub)
+    x = U.Vector(ctx, n=A.nrows)
+    s.solve(U.SparseMatrix(ctx, A), U.Vector(ctx, b), x)
+    st = s.solution_status()
+    xg = x.numpy()
+    assert st["iterates"] == so["iterates"] and st["reason"] == so["reason"]
+    np.testing.assert_allclose(s.get("lambda_max"), so["lambda_max"], rtol=1e-12)
+    assert np.array_equal(xg == lb, xo == lb) and np.array_equal(xg == ub, xo == ub)
+    assert np.linalg.norm(xg - xo) <= 1e-10 * np.linalg.norm(xo)
+
+
 def test_mprgp_unbounded_is_cg_like(ctx, oracle):
     A, b = P.poisson2d_cg(24, 2)
     s = U.MPRGP(ctx, atol=1e-10, rtol=1e-14, max_it=2000)

@@ -16,7 +16,7 @@
 // exchanges and reads through distributed shared memory: shorter exchanges, a tenth of the FP64 pipes.
 // Measured per iteration, 5-point stencil, n = 1024 / 2304 / 4096 / 6400 / 10,000 / 65,536 / 155,236 / 302,500:
 //   cluster       4.1 / 4.6 / 5.4 / 6.8 / 7.9 us
-//   CTA per SM    7.2 / 7.1 / 7.1 / 7.1 / 6.9 / 10.0 / 13.2 / 18.1 us
+//   CTA per SM    7.2 / 7.1 / 7.1 / 7.1 / 6.7 / 9.7 / 12.9 / 17.8 us
 //   kernels       21.6 / 21.7 /  - /  - / 22.9 / 22.7 / 23.7 / 29.1 us
 // Bound by the exchanges, the chain of dependent FP64 operations between them (about 70 per iteration) and, from
 // about 50,000 rows, the FP64 pipe (12 operations per row and iteration).
@@ -42,7 +42,7 @@ struct ResArgs {
     int n, rows;  // rows per CTA
     const double *b, *dinv;  // dinv null: no preconditioner
     double *x, *z, *p0, *p1;
-    void *sums;  // two GridSums
+    char *sums;  // the two exchanges' counters and partials
     CgDev *dev;
     int *kflag;
     double atol;
@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_resident(ResArgs a) {
     // the CTA's p [rows] (CL: z and two sets of p), then two arrays of blockDim.x partials (CL: and the sums' slots)
     extern __shared__ double sh[];
     __shared__ double s_sum[2], s_alpha, s_beta, s_rnorm;
+    __shared__ unsigned long long s_part[2];
     __shared__ int s_late;
     const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5;
     double *sz = sh, *sp = CL ? sh + a.rows : sh, *sq = sp + a.rows;  // CL: sp the old p, sq the new one
@@ -62,28 +63,33 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_resident(ResArgs a) {
     const int row0 = blockIdx.x * a.rows, row1 = min(a.n, row0 + a.rows);
     const bool jac = a.dinv != nullptr;  // otherwise z = r
 
-    // A sum over the grid: warp 0 adds up sa into sum 0, warp 1 (with two) sb into sum 1; then(w, sum) runs in lane 0
-    // of the warp.  The caller synchronises before it reads the sums or what then() wrote.
-    typename std::conditional<CL, ClusterSum, GridSum>::type gsum;
+    // Each sum has its own exchange, carried out by its own warp: one exchange of both by one warp measured 1 us
+    // more per iteration (its two chains of additions in one warp, and a barrier before it).
+    using Exchange = typename std::conditional<CL, ClusterExchange<1>, GridExchange<1>>::type;
+    Exchange gx;
     if constexpr (CL) {
-        gsum.init(sb + nt + (warp & 1) * ClusterSum::kDoubles, blockIdx.x, gridDim.x);
-        if (warp < 2 && lane == 0) gsum.init_barriers();
+        gx.init(sb + nt + (warp & 1) * Exchange::kDoubles, blockIdx.x, gridDim.x);
+        if (warp < 2 && lane == 0) gx.init_barriers();
         __syncthreads();
         cluster_barrier();
     } else {
-        gsum.init(a.sums, warp & 1, int(gridDim.x));
+        gx.init(a.sums + (warp & 1) * Exchange::bytes(int(gridDim.x)), int(gridDim.x));
     }
     long long ex = 0;  // exchanges of this warp's sum so far
+    // Sums over the grid: sa into sum 0 in warp 0 and, with two, sb into sum 1 in warp 1; then(w, sum) runs in lane 0 of
+    // the warp.  The caller synchronises before it reads the sums or what then() wrote.
     auto exchange = [&](bool two, auto then) {
         __syncthreads();
         if (warp < (two ? 2 : 1)) {
             const double s = warp_sum_of(warp ? sb : sa, nt);
-            double g;
-            const bool ok = gsum.exchange(ex++, s, g);
+            if (lane == 0) s_part[warp] = dbits(s);
+            __syncwarp();
+            unsigned long long g[1];
+            const bool ok = gx.exchange(ex++, s_part + warp, g);
             if (lane == 0) {
-                s_sum[warp] = g;
+                s_sum[warp] = bitsd(g[0]);
                 if (!ok) s_late = 1;
-                then(warp, g);
+                then(warp, bitsd(g[0]));
             }
         }
     };
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_resident(ResArgs a) {
             }
         }
         sa[t] = s0;
-        exchange(false, [&](int, double g) { s_alpha = rz / g; });
+        exchange(false, [&](int, double pq) { s_alpha = rz / pq; });
         __syncthreads();
         const double pAp = s_sum[0];
         alpha = s_alpha;
@@ -332,7 +338,7 @@ bool CgResident::fits(const Context &c, const Mat &A) {
     return A.nrows <= threads * (A.max_row <= kRegRow ? kMaxRpt : 2) && A.max_row <= 32;
 }
 
-size_t CgResident::sum_bytes(const Context &c) { return 2 * GridSum::bytes(c.sms); }
+size_t CgResident::sum_bytes(const Context &c) { return 2 * GridExchange<1>::bytes(c.sms); }
 
 void CgResident::run(Context &c, const Mat &A, const double *b, double *x, const double *dinv, double *z, double *p0,
                      double *p1, void *sums, CgDev *dev, double atol, long long max_it) {
@@ -357,7 +363,7 @@ void CgResident::run(Context &c, const Mat &A, const double *b, double *x, const
     a.z = z;
     a.p0 = p0;
     a.p1 = p1;
-    a.sums = sums;
+    a.sums = static_cast<char *>(sums);
     a.dev = dev;
     a.kflag = c.d_kflags() + 2;
     a.atol = atol;
@@ -365,7 +371,7 @@ void CgResident::run(Context &c, const Mat &A, const double *b, double *x, const
     UGPU_CUDA(cudaMemsetAsync(sums, 0, sum_bytes(c), c.stream));
     const bool reg = A.max_row <= kRegRow && rpt <= 2;
     const size_t smem = sizeof(double) * (size_t(rows) * (cl ? 3 : 1) + 2 * size_t(nt) +
-                                          (cl ? 2 * ClusterSum::kDoubles : 0));
+                                          (cl ? 2 * ClusterExchange<1>::kDoubles : 0));
     // one cluster has at most kClusterRows / 16 = 384 rows per CTA
     void (*f)(ResArgs) = cl         ? k_cg_resident<1, true, true>
                          : rpt == 1 ? (reg ? k_cg_resident<1, true, false> : k_cg_resident<1, false, false>)

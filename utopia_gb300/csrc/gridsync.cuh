@@ -1,12 +1,12 @@
-// Grid-wide sums inside one cooperative kernel.
+// Grid-wide sums and minima inside one kernel.
 //
-// Every CTA writes its partial sum, then adds one to the sum's counter (release); one lane per CTA polls the counter
-// until all CTAs have arrived (acquire), and a warp reads the partials and adds them in the same fixed order, so
-// all CTAs hold the same bits and take the same branches.  Three trips through L2: 2.2 us over 152 CTAs and
-// 1.8 us over 8 (448 threads each), measured in a loop of exchanges alone.  Polling the partials themselves (a
-// sentinel where none has arrived) saves a trip but has every CTA read every slot while it is written: 8 us
-// with the slots side by side, 2.9 us with one per 128-byte line.  Clusters that first add up over distributed
-// shared memory: 3.5 us.
+// Every CTA writes its partials, then adds one to a counter (release); one lane per CTA polls the counter until
+// all CTAs have arrived (acquire), and a warp reads the partials and combines them in the same fixed order,
+// so all CTAs hold the same bits and take the same branches.  Three trips through L2: 2.2 us over 152 CTAs
+// and 1.8 us over 8 (448 threads each), measured in a loop of exchanges alone.  Polling the partials themselves
+// (a sentinel where none has arrived) saves a trip but has every CTA read every slot while it is written:
+// 8 us with the slots side by side, 2.9 us with one per 128-byte line.  Clusters that first add up over
+// distributed shared memory: 3.5 us.
 //
 // Plain stores made by the CTA's threads before the __syncthreads() that precedes exchange() are visible to all
 // CTAs after the __syncthreads() that follows it, read past L1 (__ldcg).
@@ -18,26 +18,41 @@ namespace ugpu {
 
 constexpr long long kGridSpin = 4000000000ll;  // clock cycles, about 2 s
 
-// One sum's exchange: counter and partials (two sets, used in turn), zero before the launch
-struct GridSum {
-    unsigned long long *count;
-    double *part;  // [2][G]
-    int G;         // CTAs
-    static __host__ __device__ constexpr size_t bytes(int G) { return 128 + sizeof(double) * 2 * size_t(G); }
-    __device__ __forceinline__ void init(void *base, int d, int ctas) {  // the d-th sum of a buffer of several
-        char *b = static_cast<char *>(base) + d * bytes(ctas);
-        count = reinterpret_cast<unsigned long long *>(b);
-        part = reinterpret_cast<double *>(b + 128);
+// The NV values of an exchange are 64-bit patterns: doubles to be added, or (bits of MIN) order keys whose
+// minimum is wanted.
+template <int NV, int MIN>
+struct Values {
+    static __device__ __forceinline__ unsigned long long none(int i) { return (MIN >> i & 1) ? ~0ull : 0ull; }
+    static __device__ __forceinline__ unsigned long long both(int i, unsigned long long a, unsigned long long b) {
+        if (MIN >> i & 1) return a < b ? a : b;
+        return (unsigned long long)__double_as_longlong(__longlong_as_double((long long)a) +
+                                                        __longlong_as_double((long long)b));
+    }
+};
+__device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned long long)__double_as_longlong(v); }
+__device__ __forceinline__ double bitsd(unsigned long long b) { return __longlong_as_double((long long)b); }
+
+// Counter and partials (two sets, used in turn) of one kind of exchange, zero before the launch
+template <int NV, int MIN = 0>
+struct GridExchange {
+    using V = Values<NV, MIN>;
+    unsigned long long *count, *part;  // part: [2][NV][G]
+    int G;                             // CTAs
+    static constexpr size_t bytes(int G) { return 128 + sizeof(unsigned long long) * 2 * NV * size_t(G); }
+    __device__ __forceinline__ void init(char *base, int ctas) {
+        count = reinterpret_cast<unsigned long long *>(base);
+        part = reinterpret_cast<unsigned long long *>(base + 128);
         G = ctas;
     }
-    // One full warp: the k-th exchange (k = 0, 1, ...) of this sum, v in lane 0.  False if a CTA did not arrive
-    // in time.
-    __device__ __forceinline__ bool exchange(long long k, double v, double &sum) const {
+    // One full warp: the k-th exchange (k = 0, 1, ...) of the CTA's NV values in shared memory; out in every lane.
+    // False if a CTA did not arrive in time.
+    __device__ __forceinline__ bool exchange(long long k, const unsigned long long *v, unsigned long long (&out)[NV]) const {
         const int lane = threadIdx.x & 31;
-        double *p = part + int64_t(k & 1) * G;
+        unsigned long long *p = part + int64_t(k & 1) * NV * G;
+        if (lane < NV) __stcg(p + lane * G + blockIdx.x, v[lane]);
+        __syncwarp();
         int ok = 1;
         if (lane == 0) {
-            __stcg(p + blockIdx.x, v);
             asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
             const unsigned long long want = (unsigned long long)(k + 1) * (unsigned long long)G;
             const long long t0 = clock64();
@@ -52,38 +67,49 @@ struct GridSum {
             }
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
-        double s = 0.0;
-        for (int j0 = 0; j0 < G; j0 += 32 * 8) {  // up to eight partials per lane in flight
-            double t[8];
+        unsigned long long s[NV];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int j = j0 + 32 * q + lane;
-                t[q] = j < G ? __ldcg(p + j) : 0.0;
-            }
+        for (int i = 0; i < NV; ++i) s[i] = V::none(i);
+        for (int j0 = 0; j0 < G; j0 += 32 * 5) {  // up to five partials per lane and value in flight
             const int live = (G - j0 + 31) / 32;  // groups of 32 that hold partials
+            unsigned long long t[NV][5];
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (q < live) s += t[q];
+            for (int i = 0; i < NV; ++i)
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {
+                    const int j = j0 + 32 * q + lane;
+                    t[i][q] = j < G ? __ldcg(p + i * G + j) : V::none(i);
+                }
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+                if (q < live)
+#pragma unroll
+                    for (int i = 0; i < NV; ++i) s[i] = V::both(i, s[i], t[i][q]);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        sum = s;
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) s[i] = V::both(i, s[i], __shfl_xor_sync(0xffffffffu, s[i], o));
+#pragma unroll
+        for (int i = 0; i < NV; ++i) out[i] = s[i];
         return ok != 0;
     }
 };
 
-// The same within one cluster of at most 16 CTAs: every CTA's warp stores its partial into every CTA's shared
+// The same within one cluster of at most 16 CTAs: every CTA's warp stores its partials into every CTA's shared
 // memory (st.async) and counts the arriving bytes on its own mbarrier.  0.6 us over 16 CTAs where the exchange
 // through L2 takes 1.8 us even over 8; the cluster barrier with the same stores takes 0.9-1.6 us.  Data that the
 // CTA's threads stored to shared memory before the preceding __syncthreads() may be read by the cluster's
 // other CTAs after the following one.
-struct ClusterSum {
-    uint32_t slots, bars;  // shared addresses: [2][16] doubles, [2] mbarriers
+template <int NV, int MIN = 0>
+struct ClusterExchange {
+    using V = Values<NV, MIN>;
+    uint32_t slots, bars;  // shared addresses: [2][NV][16] 64-bit slots, [2] mbarriers
     uint32_t rank, size;
-    static constexpr int kDoubles = 2 * 16 + 2;  // shared doubles of one sum
+    static constexpr int kDoubles = 2 * NV * 16 + 2;  // shared 8-byte words
     __device__ __forceinline__ void init(double *shared, uint32_t r, uint32_t n) {
         slots = uint32_t(__cvta_generic_to_shared(shared));
-        bars = slots + 2 * 16 * 8;
+        bars = slots + 2 * NV * 16 * 8;
         rank = r;
         size = n;
     }
@@ -91,21 +117,22 @@ struct ClusterSum {
         for (int i = 0; i < 2; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // one full warp, v in lane 0
-    __device__ __forceinline__ bool exchange(long long k, double v, double &sum) const {
+    __device__ __forceinline__ bool exchange(long long k, const unsigned long long *v, unsigned long long (&out)[NV]) const {
         const uint32_t lane = threadIdx.x & 31, b = uint32_t(k & 1), parity = uint32_t(k >> 1) & 1u;
         if (lane == 0)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * b), "r"(8u * size)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * b), "r"(8u * NV * size)
                          : "memory");
-        v = __shfl_sync(0xffffffffu, v, 0);
+        __syncwarp();
         if (lane < size) {
             uint32_t ra, rb;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(slots + (b * 16 + rank) * 8), "r"(lane));
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(slots + (b * NV * 16 + rank) * 8), "r"(lane));
             asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bars + 8 * b), "r"(lane));
             asm volatile("fence.acq_rel.cluster;" ::: "memory");
-            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(ra),
-                         "l"(__double_as_longlong(v)), "r"(rb)
-                         : "memory");
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(ra + i * 128),
+                             "l"(v[i]), "r"(rb)
+                             : "memory");
         }
         uint32_t ok = 0;
         const long long t0 = clock64();
@@ -119,13 +146,22 @@ struct ClusterSum {
                 : "memory");
             if (ok || clock64() - t0 > kGridSpin) break;
         }
-        unsigned long long t = 0ull;
-        if (lane < size)
-            asm volatile("ld.shared::cta.u64 %0, [%1];" : "=l"(t) : "r"(slots + (b * 16 + lane) * 8) : "memory");
-        double s = __longlong_as_double((long long)t);
+        unsigned long long s[NV];
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        sum = __shfl_sync(0xffffffffu, s, 0);
+        for (int i = 0; i < NV; ++i) {
+            s[i] = V::none(i);
+            if (lane < size)
+                asm volatile("ld.shared::cta.u64 %0, [%1];"
+                             : "=l"(s[i])
+                             : "r"(slots + ((b * NV + i) * 16 + lane) * 8)
+                             : "memory");
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) s[i] = V::both(i, s[i], __shfl_xor_sync(0xffffffffu, s[i], o));
+#pragma unroll
+        for (int i = 0; i < NV; ++i) out[i] = __shfl_sync(0xffffffffu, s[i], 0);
         return __all_sync(0xffffffffu, ok != 0);
     }
 };

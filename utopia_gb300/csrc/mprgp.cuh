@@ -1,0 +1,33 @@
+// MPRGP's device state and its resident form (mprgp_resident.cu).
+#pragma once
+#include "internal.cuh"
+
+namespace ugpu {
+
+struct QpDev {
+    double qa0, qa1;              // the iteration's product s -> A s: (s, A s), (s, g); s = p or beta
+    double neg_bsc;               // -beta_sc of the pending direction p = fi - beta_sc p (0: p = fi)
+    unsigned long long amin;      // key (qp_key) of alpha_f = min step bound, reset after each use
+    double alpha_cg, alpha_f, beta_sc;
+    double beta_beta, fi_fi, gnorm, gnorm0;
+    long long it, iterates;
+    int done, reason, converged;
+    int gate_cg, gate_prop, gate_exp;   // branch of the current iteration
+    int step;                           // 0: CG step, 1: expansion step
+    double lambda;                      // the power method's estimate (resident form)
+};
+
+// A solve of small problems as one kernel (work on c.stream).
+// fi, beta, p0, p1: n doubles each; sums: sum_bytes(); dev receives the final state.
+struct MprgpResident {
+    static bool fits(const Context &c, const Mat &A);
+    // Whether run() makes the power-method estimate itself (lambda = 0): up to two rows per thread.  On larger
+    // problems its 0.6 ms of host round trips is nothing beside the solve.
+    static bool own_power_method(const Context &c, const Mat &A);
+    static size_t sum_bytes(const Context &c);
+    static void run(Context &c, const Mat &A, const double *b, double *x, const double *lb, const double *ub, double *fi,
+                    double *beta, double *p0, double *p1, void *sums, QpDev *dev, double atol, double rtol,
+                    long long max_it, double lambda, double eig_tol, long long eig_max_it);
+};
+
+}  // namespace ugpu

@@ -6,7 +6,8 @@
 // branch decisions of every iteration (proportional vs proportioning, CG vs expansion
 // step, negative curvature, convergence) are taken on the device by the last CTA of
 // the kernel that produces the deciding dots; the kernels of the branches that are
-// not taken return at once, so a batch of iterations runs without host round trips.
+// not taken return at once, so a batch of iterations runs without host round trips.  Small problems run the same
+// loop in one kernel (mprgp_resident.cu).
 //
 // ProjectedGaussSeidel mirrors utopia::ProjectedGaussSeidel::apply/step
 // (utopia_ProjectedGaussSeidel.hpp:71-112,197-318) with the lexicographic row loop
@@ -19,6 +20,8 @@
 
 #include "abi_util.cuh"
 #include "device_util.cuh"
+#include "mprgp.cuh"
+#include "qp_device.cuh"
 #include "solver.cuh"
 
 namespace ugpu {
@@ -27,31 +30,6 @@ namespace {
 
 #define QP_LOOP(i, n) \
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < (n); i += int64_t(gridDim.x) * blockDim.x)
-
-struct QpDev {
-    double qa0, qa1;              // the iteration's product s -> A s: (s, A s), (s, g); s = p or beta
-    double neg_bsc;               // -beta_sc of the pending direction p = fi - beta_sc p (0: p = fi)
-    unsigned long long amin;      // key (qp_key) of alpha_f = min step bound, reset after each use
-    double alpha_cg, alpha_f, beta_sc;
-    double beta_beta, fi_fi, gnorm, gnorm0;
-    long long it, iterates;
-    int done, reason, converged;
-    int gate_cg, gate_prop, gate_exp;   // branch of the current iteration
-    int step;                           // 0: CG step, 1: expansion step
-};
-
-// the predicates of MPRGP / VariableBoundSolverInterface with their comparisons on the integer
-// pipes (device_util.cuh: exact for non-NaN bounds and iterates)
-__device__ __forceinline__ double proj(double l, double u, double x) {
-    const long long xk = dkey(x);
-    return (dkey(l) >= xk) ? l : ((dkey(u) <= xk) ? u : x);
-}
-__device__ __forceinline__ double phi(double l, double u, double x, double g) { return (dlt(l, x) && dlt(x, u)) ? g : 0.0; }
-// (|l - x| < 1e-14) ? min(0, g) : ((|u - x| < 1e-14) ? max(0, g) : 0)
-__device__ __forceinline__ double chopped(double l, double u, double x, double g) {
-    if (dabs_lt(l - x, 1e-14)) return dmin0(g);
-    return dabs_lt(u - x, 1e-14) ? dmax0(g) : 0.0;
-}
 
 __device__ __forceinline__ void qp_stop(QpDev *d, int reason, int converged) {
     d->done = 1;
@@ -613,6 +591,20 @@ public:
         st = ugpu_solution_status{};
         const double *lb, *ub;
         bounds(n, &lb, &ub);
+        // Small problems: the whole solve as one resident kernel, with and without use_graphs (mprgp_resident.cu)
+        if (MprgpResident::fits(*ctx, *op)) {
+            if (!sums_.ptr) sums_.alloc(MprgpResident::sum_bytes(*ctx));
+            const double lambda = MprgpResident::own_power_method(*ctx, *op) ? 0.0 : power_method();
+            MprgpResident::run(*ctx, *op, rhs.as<double>(), x.as<double>(), lb, ub, fi_.as<double>(),
+                               beta_.as<double>(), p_.as<double>(), Ap_.as<double>(), sums_.ptr, dev_.as<QpDev>(),
+                               get("atol"), get("rtol"), (long long)get("max_it"), lambda, get("eig_comp_tol"),
+                               (long long)get("power_method_max_it"));
+            UGPU_CUDA(cudaMemcpyAsync(host_, dev_.ptr, sizeof(QpDev), cudaMemcpyDeviceToHost, ctx->stream));
+            ctx->check_kernel_flags();
+            prm["lambda_max"] = lambda_max = host_->lambda;
+            finish(t0, l0);
+            return;
+        }
         lambda_max = power_method();
         prm["lambda_max"] = lambda_max;
         alpha_bar_ = 1.95 / lambda_max;
@@ -634,6 +626,18 @@ public:
         rhs_ = rhs.as<double>();
         run_loop(loop_, key_, {x.data(), lb, ub, rhs_}, alpha_bar_, [&] { iteration(x.as<double>(), lb, ub); },
                  &dev_.as<QpDev>()->done, dev_, host_, sizeof(QpDev));
+        finish(t0, l0);
+    }
+
+private:
+    Buffer fi_, beta_, p_, Ap_, g_, h1_, h2_, dev_, part_, cnt_, sums_;
+    QpDev *host_ = nullptr;
+    double alpha_bar_ = 1;
+    const double *rhs_ = nullptr;
+    DeviceLoop loop_;
+    LoopKey key_;
+
+    void finish(double t0, int64_t l0) {
         st.iterates = host_->iterates;
         st.gradient_norm = host_->gnorm;
         st.relative_gradient_norm = host_->gnorm0 > 0 ? host_->gnorm / host_->gnorm0 : 1;
@@ -644,14 +648,6 @@ public:
         st.execution_time = now_s() - t0;
         st.kernel_launches = ctx->launches - l0;
     }
-
-private:
-    Buffer fi_, beta_, p_, Ap_, g_, h1_, h2_, dev_, part_, cnt_;
-    QpDev *host_ = nullptr;
-    double alpha_bar_ = 1;
-    const double *rhs_ = nullptr;
-    DeviceLoop loop_;
-    LoopKey key_;
 
     void final_kernel(double *x, const double *lb, const double *ub, int first) {
         const int64_t n = op->nrows;
