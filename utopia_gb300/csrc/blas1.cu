@@ -121,35 +121,50 @@ __device__ __forceinline__ double load_any(const void *p, int dt, int64_t i) {
 
 // Fused multi-dot with a deterministic two-stage reduction: every CTA reduces a fixed
 // strided subset in a fixed order; the last CTA to finish sums the CTA partials in
-// CTA order and writes out[k].  MODE 0: all operands FP64, 1: all FP32, 2: mixed.
-template <int MODE>
+// CTA order and writes out[k].  MODE 0: all operands FP64, 1: all FP32, 2: mixed.  ND: the number of dots, or
+// kMaxDots for any (args.nd).  With one or two dots four strides' operands are loaded before they are used, in the
+// same order of additions: a loop of single loads left each thread a chain of memory latencies
+// (one dot of 2 M elements 20 us, 8 us so).  done (may be null): nothing happens when *done != 0.
+template <int MODE, int ND>
 __global__ void __launch_bounds__(kBlock) k_dots(int64_t n, DotArgs args, double *partials, double *out,
-                                                unsigned int *counter) {
-    const int nd = args.nd;
-    double acc[kMaxDots];
+                                                unsigned int *counter, const int *done) {
+    if (done && *done) return;
+    const int nd = ND < kMaxDots ? ND : args.nd;
+    double acc[ND];
 #pragma unroll
-    for (int k = 0; k < kMaxDots; ++k) acc[k] = 0.0;
+    for (int k = 0; k < ND; ++k) acc[k] = 0.0;
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += stride) {
+    auto operand = [&](const void *p, int dt, int64_t i) {
+        if (MODE == 0) return static_cast<const double *>(p)[i];
+        if (MODE == 1) return double(static_cast<const float *>(p)[i]);
+        return load_any(p, dt, i);
+    };
+    int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (ND < kMaxDots) {
+        constexpr int U = 4;
+        for (; i + (U - 1) * stride < n; i += U * stride) {
+            double a[U][ND], b[U][ND];
 #pragma unroll
-        for (int k = 0; k < kMaxDots; ++k) {
-            if (k < nd) {
-                double a, b;
-                if (MODE == 0) {
-                    a = static_cast<const double *>(args.a[k])[i];
-                    b = static_cast<const double *>(args.b[k])[i];
-                } else if (MODE == 1) {
-                    a = double(static_cast<const float *>(args.a[k])[i]);
-                    b = double(static_cast<const float *>(args.b[k])[i]);
-                } else {
-                    a = load_any(args.a[k], args.dtype_a[k], i);
-                    b = load_any(args.b[k], args.dtype_b[k], i);
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < ND; ++k) {
+                    a[u][k] = operand(args.a[k], args.dtype_a[k], i + u * stride);
+                    b[u][k] = operand(args.b[k], args.dtype_b[k], i + u * stride);
                 }
-                acc[k] = fma(a, b, acc[k]);
-            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int k = 0; k < ND; ++k) acc[k] = fma(a[u][k], b[u][k], acc[k]);
         }
     }
-    block_reduce_store<kMaxDots>(acc, nd, partials, gridDim.x, blockIdx.x);
+#pragma unroll 1
+    for (; i < n; i += stride) {
+#pragma unroll
+        for (int k = 0; k < ND; ++k)
+            if (k < nd)
+                acc[k] = fma(operand(args.a[k], args.dtype_a[k], i), operand(args.b[k], args.dtype_b[k], i), acc[k]);
+    }
+    block_reduce_store<ND>(acc, nd, partials, gridDim.x, blockIdx.x);
     finish_last_block(nd, partials, gridDim.x, out, counter);
 }
 
@@ -256,21 +271,31 @@ int stream_grid(const Context &ctx, int64_t n) {
     return int(g);
 }
 
+// mode: the operands' types (k_dots' MODE)
+static void run_dots(int mode, int64_t n, const DotArgs &args, double *partials, double *out, unsigned int *counter,
+                     const int *done, cudaStream_t stream) {
+    const int g = reduce_grid(n);
+    auto run = [&](auto kern) { kern<<<g, kBlock, 0, stream>>>(n, args, partials, out, counter, done); };
+    auto by_count = [&](auto m) {
+        constexpr int M = decltype(m)::value;
+        if (args.nd == 1) run(k_dots<M, 1>);
+        else if (args.nd == 2) run(k_dots<M, 2>);
+        else run(k_dots<M, kMaxDots>);
+    };
+    if (mode == 0) by_count(std::integral_constant<int, 0>{});
+    else if (mode == 1) by_count(std::integral_constant<int, 1>{});
+    else by_count(std::integral_constant<int, 2>{});
+}
+
 void launch_dots_into(Context &ctx, int64_t n, const DotArgs &args, double *d_out, double *partials,
-                      unsigned int *counter) {
+                      unsigned int *counter, const int *done) {
     UGPU_CHECK(args.nd >= 1 && args.nd <= kMaxDots, UGPU_ERR_ARG, "1..8 dots per pass");
     bool all64 = true, all32 = true;
     for (int k = 0; k < args.nd; ++k) {
         all64 &= args.dtype_a[k] == UGPU_F64 && args.dtype_b[k] == UGPU_F64;
         all32 &= args.dtype_a[k] == UGPU_F32 && args.dtype_b[k] == UGPU_F32;
     }
-    int g = reduce_grid(n);
-    if (all64)
-        k_dots<0><<<g, kBlock, 0, ctx.stream>>>(n, args, partials, d_out, counter);
-    else if (all32)
-        k_dots<1><<<g, kBlock, 0, ctx.stream>>>(n, args, partials, d_out, counter);
-    else
-        k_dots<2><<<g, kBlock, 0, ctx.stream>>>(n, args, partials, d_out, counter);
+    run_dots(all64 ? 0 : all32 ? 1 : 2, n, args, partials, d_out, counter, done, ctx.stream);
     ctx.launches++;
     UGPU_LAUNCH_CHECK();
 }
@@ -732,13 +757,8 @@ extern "C" int ugpu_dots_noalloc(int k, const void *const *a, const void *const 
         all64 &= args.dtype_a[i] == UGPU_F64 && args.dtype_b[i] == UGPU_F64;
         all32 &= args.dtype_a[i] == UGPU_F32 && args.dtype_b[i] == UGPU_F32;
     }
-    const int g = reduce_grid(n);  // at most kRedBlocks CTAs: the partials fit the scratch
-    if (all64)
-        k_dots<0><<<g, kBlock, 0, s>>>(n, args, partials, d_out, ticket);
-    else if (all32)
-        k_dots<1><<<g, kBlock, 0, s>>>(n, args, partials, d_out, ticket);
-    else
-        k_dots<2><<<g, kBlock, 0, s>>>(n, args, partials, d_out, ticket);
+    // at most kRedBlocks CTAs: the partials fit the scratch
+    run_dots(all64 ? 0 : all32 ? 1 : 2, n, args, partials, d_out, ticket, nullptr, s);
     UGPU_CUDA(cudaGetLastError());
     UGPU_ABI_END(nullptr)
 }

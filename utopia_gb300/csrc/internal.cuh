@@ -234,7 +234,7 @@ struct DotArgs {
 };
 void launch_dots(Context &ctx, int64_t n, const DotArgs &args, double *d_out);
 void launch_dots_into(Context &ctx, int64_t n, const DotArgs &args, double *d_out, double *partials,
-                      unsigned int *counter);
+                      unsigned int *counter, const int *done = nullptr);
 void host_dots(Context &ctx, int64_t n, const DotArgs &args, double *out);
 int reduce_grid(int64_t n);
 int stream_grid(const Context &ctx, int64_t n);

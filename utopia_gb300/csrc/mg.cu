@@ -41,14 +41,96 @@ struct GlibcRand {
         }
         for (int k = 0; k < 310; ++k) next();
     }
-    int32_t next() {
+    uint32_t next() {  // the 32-bit state word; rand() returns it shifted right by one
         ring[f] += ring[b];
-        int32_t out = int32_t(ring[f] >> 1);
+        const uint32_t out = ring[f];
         f = (f + 1) % 31;
         b = (b + 1) % 31;
         return out;
     }
 };
+
+// The start vectors on the device.  The state words obey x_n = x_{n-3} + x_{n-31} (mod 2^32), so x_{n+m} is the
+// combination of x_n .. x_{n+30} with the coefficients of z^m mod (z^31 - z^28 - 1) over the integers mod 2^32.  Every
+// warp jumps to its own position m (a product of the tabulated powers z^(2^k)) and goes on from there 31
+// words at a time: word i of the next window is a sum of every third word of this one.  The values are those of
+// the sequential generator, which took 9 ms on the host for the 2.4 million rows of a 128^3 hierarchy, with
+// the copy to the device; this takes 0.26 ms.
+constexpr int kRandWords = 31;
+constexpr int kRandChunk = 64 * kRandWords;  // words per warp: the jump costs as much as about 100 windows
+struct RandTable {
+    uint32_t base[2 * kRandWords - 1];   // x_0 .. x_60
+    uint32_t pow[32][kRandWords];        // z^(2^k)
+    explicit RandTable(uint32_t seed) {
+        GlibcRand g(seed);
+        for (auto &x : base) x = g.next();
+        uint32_t a[kRandWords] = {0, 1};  // z
+        for (int k = 0; k < 32; ++k) {
+            for (int i = 0; i < kRandWords; ++i) pow[k][i] = a[i];
+            uint32_t c[2 * kRandWords - 1] = {};
+            for (int i = 0; i < kRandWords; ++i)
+                for (int j = 0; j < kRandWords; ++j) c[i + j] += a[i] * a[j];
+            for (int d = 2 * kRandWords - 2; d >= kRandWords; --d) {
+                c[d - 3] += c[d];
+                c[d - 31] += c[d];
+            }
+            for (int i = 0; i < kRandWords; ++i) a[i] = c[i];
+        }
+    }
+};
+
+// out_i = rand_{first + i} / RAND_MAX + 1, i < n
+__global__ void __launch_bounds__(128) k_pm_start(const __grid_constant__ RandTable t, uint32_t first, int64_t n,
+                                                  double *out) {
+    __shared__ uint32_t s_a[4][kRandWords], s_c[4][2 * kRandWords];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t begin = (blockIdx.x * int64_t(4) + w) * kRandChunk;
+    if (begin >= n) return;
+    uint32_t *a = s_a[w], *c = s_c[w];
+    const uint32_t m = first + uint32_t(begin);
+    if (lane < kRandWords) a[lane] = lane == 0 ? 1u : 0u;
+    __syncwarp();
+    for (int k = 0; k < 32; ++k) {
+        if (!(m >> k & 1u)) continue;
+        // a = a z^(2^k): coefficients `lane` and `lane + 31` of the product, then degrees 60 .. 31 folded three at a time
+        uint32_t p0 = 0, p1 = 0;
+        for (int i = 0; i < kRandWords; ++i) {
+            const uint32_t x = a[i];
+            const int j0 = lane - i, j1 = lane + kRandWords - i;
+            if (j0 >= 0 && lane < kRandWords) p0 += x * t.pow[k][j0];
+            if (j1 < kRandWords) p1 += x * t.pow[k][j1];
+        }
+        if (lane < kRandWords) {
+            c[lane] = p0;
+            c[lane + kRandWords] = p1;
+        }
+        __syncwarp();
+        for (int d = 2 * kRandWords - 2; d >= kRandWords; d -= 3) {
+            if (lane < 3) {
+                c[d - lane - 3] += c[d - lane];
+                c[d - lane - 31] += c[d - lane];
+            }
+            __syncwarp();
+        }
+        if (lane < kRandWords) a[lane] = c[lane];
+        __syncwarp();
+    }
+    uint32_t x = 0;
+    if (lane < kRandWords)
+        for (int j = 0; j < kRandWords; ++j) x += a[j] * t.base[lane + j];
+    const int64_t end = min(n, begin + kRandChunk);
+    for (int64_t i = begin; i < end; i += kRandWords) {
+        if (lane < kRandWords && i + lane < end) out[i + lane] = (double(int32_t(x >> 1)) / 2147483647.0) + 1;
+        const uint32_t last = __shfl_sync(0xffffffffu, x, 28 + lane % 3);
+        uint32_t s = x;
+#pragma unroll
+        for (int o = 3; o < kRandWords; o *= 2) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        x = s + last;
+    }
+}
 
 // MultiLevelMask::generate_mask_from_matrix: m_i = 0 if row i has an off-diagonal |a| > tol, else 1
 template <class V>
@@ -80,7 +162,9 @@ __global__ void k_mask_final(const double *m, int64_t n, T *out, unsigned long l
         out[i] = T(v);
         z += (v == 0.0);
     }
-    atomicAdd(zeros, z);
+    // one atomic per warp that saw zeros: one per thread took 150 us on 2 M rows without any
+    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    if (z && (threadIdx.x & 31) == 0) atomicAdd(zeros, z);
 }
 
 // PowerMethod loop body (utopia_PowerMethod.hpp:122-146) after y = A v and dot = (y, y):
@@ -290,11 +374,10 @@ public:
         }
         make_masks();
         // Multigrid::update(): smoothers of levels 1..L-1 in order, then the coarse solver
-        GlibcRand rng(uint32_t(get("rand_seed")));
         const int sm = int(get("smoother"));
         for (int l = 1; l < L; ++l) setup_smoother(l, sm);
         if (sm == 1) {
-            power_methods(rng);
+            power_methods();
             for (int l = 1; l < L; ++l) chebyshev_coefficients(levels_[l]);
         }
         UGPU_CHECK(coarse_.factor(*levels_[0].A64), UGPU_ERR_NOT_SPD,
@@ -522,15 +605,12 @@ private:
     // levels are updated one after the other); the levels' iterations are independent, so they
     // run concurrently on one stream per level (each with its own reduction scratch), joined
     // back into the context's stream before the estimates are read.
-    void power_methods(GlibcRand &rng) {
+    void power_methods() {
         const int L = n_levels();
         const double tol = get("power_method_tol");
         const long long max_it = (long long)get("power_method_max_it");
-        std::vector<std::vector<double>> h(L);
-        for (int l = 1; l < L; ++l) {
-            h[l].resize(size_t(levels_[l].n));
-            for (auto &x : h[l]) x = (double(rng.next()) / 2147483647.0) + 1;
-        }
+        const RandTable rand(uint32_t(get("rand_seed")));
+        uint32_t drawn = 0;
         if (pm_.size() < size_t(L)) pm_.resize(L);
         while (pm_streams_.size() < size_t(L)) {
             cudaStream_t st;
@@ -579,8 +659,12 @@ private:
             long long *itp = reinterpret_cast<long long *>(done + 2);
             const double *v = ps.v.as<double>(), *w = ps.w.as<double>();
             UGPU_CUDA(cudaMemsetAsync(ps.st.ptr, 0, ps.st.bytes, ctx->stream));
-            if (n) UGPU_CUDA(cudaMemcpyAsync(ps.v.ptr, h[l].data(), sizeof(double) * n, cudaMemcpyHostToDevice,
-                                             ctx->stream));
+            if (n) {
+                const int64_t warps = (n + kRandChunk - 1) / kRandChunk;
+                k_pm_start<<<unsigned((warps + 3) / 4), 128, 0, ctx->stream>>>(rand, drawn, n, ps.v.as<double>());
+                ctx->launches++;
+                drawn += uint32_t(n);
+            }
             DotArgs d{};
             d.nd = 1;
             d.dtype_a[0] = d.dtype_b[0] = UGPU_F64;
@@ -600,7 +684,7 @@ private:
                 a.done = done;
                 launch_spmv(*ctx, *lv.A64, a);
                 d.a[0] = d.b[0] = w;
-                launch_dots_into(*ctx, n, d, dst, ps.part.as<double>(), ps.cnt.as<unsigned int>());
+                launch_dots_into(*ctx, n, d, dst, ps.part.as<double>(), ps.cnt.as<unsigned int>(), done);
                 k_pm_check<<<1, 1, 0, ctx->stream>>>(dst, done, itp, tol, max_it);
                 k_pm_scale<<<g, kBlock, 0, ctx->stream>>>(n, w, dst + 1, done + 1, ps.v.as<double>());
                 ctx->launches += 2;
