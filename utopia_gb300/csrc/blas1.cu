@@ -1,6 +1,8 @@
 // Context, vectors, BLAS-1 kernels and deterministic reductions.
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "abi_util.cuh"
 #include "device_util.cuh"
@@ -8,6 +10,31 @@
 namespace ugpu {
 
 thread_local std::string g_last_error;
+thread_local const std::shared_ptr<StreamRef> *PoolScope::current = nullptr;
+
+// The device's pool (one per process): keeps at most a sixteenth of the device's memory beyond what is in use, the
+// size of a 192^3 hierarchy several times over.  Null where the device has none: plain allocations then.
+static cudaMemPool_t device_pool(int dev, size_t memory) {
+    static std::mutex mutex;
+    static std::map<int, cudaMemPool_t> pools;
+    std::lock_guard<std::mutex> lock(mutex);
+    auto it = pools.find(dev);
+    if (it != pools.end()) return it->second;
+    int supported = 0;
+    cudaMemPool_t pool = nullptr;
+    UGPU_CUDA(cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, dev));
+    if (supported) {
+        cudaMemPoolProps p{};
+        p.allocType = cudaMemAllocationTypePinned;
+        p.location.type = cudaMemLocationTypeDevice;
+        p.location.id = dev;
+        UGPU_CUDA(cudaMemPoolCreate(&pool, &p));
+        uint64_t keep = uint64_t(memory / 16);
+        UGPU_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    pools[dev] = pool;
+    return pool;
+}
 
 Context::Context(int dev) : device(dev) {
     int count = 0;
@@ -17,7 +44,10 @@ Context::Context(int dev) : device(dev) {
     cudaDeviceProp prop;
     UGPU_CUDA(cudaGetDeviceProperties(&prop, dev));
     sms = prop.multiProcessorCount;
-    UGPU_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    stream_ref = std::make_shared<StreamRef>();
+    UGPU_CUDA(cudaStreamCreateWithFlags(&stream_ref->s, cudaStreamNonBlocking));
+    stream = stream_ref->s;
+    stream_ref->pool = device_pool(dev, prop.totalGlobalMem);
     partials.alloc(sizeof(double) * kMaxDots * kRedBlocks);
     scalars.alloc(sizeof(double) * 256);
     counters.alloc(sizeof(unsigned int) * 64);
@@ -49,10 +79,8 @@ void Context::check_kernel_flags() {
 }
 
 Context::~Context() {
-    if (stream) {
-        cudaStreamSynchronize(stream);
-        cudaStreamDestroy(stream);
-    }
+    if (stream) cudaStreamSynchronize(stream);
+    if (stream_ref && stream_ref->pool) cudaMemPoolTrimTo(stream_ref->pool, 0);
     if (host_scalars) cudaFreeHost(host_scalars);
 }
 

@@ -96,6 +96,7 @@ int ugpu_mg_set_transfer_operators(ugpu_solver *mg, int n, const ugpu_mat *const
     UGPU_ABI_BEGIN
     UGPU_REQUIRE(mg);
     UGPU_CHECK(n >= 1 && interpolations, UGPU_ERR_ARG, "at least one interpolation operator");
+    PoolScope pooled(mg->impl->ctx->stream_ref);
     std::vector<const Mat *> P;
     for (int i = 0; i < n; ++i) {
         UGPU_CHECK(interpolations[i], UGPU_ERR_ARG, "null interpolation operator");
@@ -153,6 +154,7 @@ int ugpu_solver_update(ugpu_solver *s, const ugpu_mat *A) {
     UGPU_ABI_BEGIN
     UGPU_REQUIRE(s);
     UGPU_REQUIRE(A);
+    PoolScope pooled(s->impl->ctx->stream_ref);
     s->impl->update(&A->impl);
     UGPU_CUDA(cudaStreamSynchronize(s->impl->ctx->stream));
     UGPU_ABI_END(s ? s->impl->ctx : nullptr)
@@ -163,6 +165,7 @@ int ugpu_solver_apply(ugpu_solver *s, const ugpu_vec *rhs, ugpu_vec *x) {
     UGPU_REQUIRE(s);
     UGPU_REQUIRE(rhs);
     UGPU_REQUIRE(x);
+    PoolScope pooled(s->impl->ctx->stream_ref);
     s->impl->apply(rhs->impl, x->impl);
     s->impl->ctx->check_kernel_flags();
     UGPU_ABI_END(s ? s->impl->ctx : nullptr)
