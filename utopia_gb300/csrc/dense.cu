@@ -62,30 +62,25 @@ __global__ void k_densify(const int32_t *rp, const int32_t *ci, const V *cv, int
     }
 }
 
-// 1 / v for v > 0 to FP64 rounding: an FP32 estimate of the significand's reciprocal and one third-order
-// step, three FP64 instructions in a chain (the pivots of a block follow one another).
+// 1 / v for v > 0 to FP64 rounding: the approximation instruction's estimate (about 20 bits) and one third-order
+// step of Householder's iteration, three FP64 instructions in a chain (the pivots of a block follow one another).
 __device__ __forceinline__ double rcp_pivot(double v) {
-    const long long b = __double_as_longlong(v);
-    const int e = int(b >> 52) - 1023;
-    if (e < -1020 || e > 1020) return 1.0 / v;  // subnormals, infinity, NaN, reciprocals near them
-    const double m = __longlong_as_double(b - e * (1ll << 52));  // in [1, 2)
-    const double r0 = f2d_bits(1.0f / d2f_bits(m));
-    const double d = fma(-m, r0, 1.0);
-    const double r = fma(r0, fma(d, d, d), r0);
-    return __longlong_as_double(__double_as_longlong(r) - e * (1ll << 52));
+    const int e = (__double2hiint(v) >> 20) - 1023;
+    if (e < -1000 || e > 1000) return 1.0 / v;  // subnormals, infinity, NaN, reciprocals near them
+    double r0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(v));
+    const double d = fma(-v, r0, 1.0);
+    return fma(r0, fma(d, d, d), r0);
 }
 
 // 1 / sqrt(v) likewise, five FP64 instructions.
 __device__ __forceinline__ double rsqrt_pivot(double v) {
-    const long long b = __double_as_longlong(v);
-    const int e = int(b >> 52) - 1023;
-    if (e < -1020 || e > 1020) return 1.0 / sqrt(v);
-    const int h = e >> 1;                                              // v = m 4^h
-    const double m = __longlong_as_double(b - 2 * h * (1ll << 52));    // in [1, 4)
-    const double r0 = f2d_bits(rsqrtf(d2f_bits(m)));
-    const double d = fma(-(m * r0), r0, 1.0);
-    const double r = fma(r0 * d, fma(d, 0.375, 0.5), r0);
-    return __longlong_as_double(__double_as_longlong(r) - h * (1ll << 52));
+    const int e = (__double2hiint(v) >> 20) - 1023;
+    if (e < -1000 || e > 1000) return 1.0 / sqrt(v);
+    double r0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(v));
+    const double d = fma(-(v * r0), r0, 1.0);
+    return fma(r0 * d, fma(d, 0.375, 0.5), r0);
 }
 
 // Cholesky of the kb x kb diagonal block at (k0, k0) of A (A = L L^T) and Y = L^-1, into Y's block.  Column c
@@ -97,8 +92,9 @@ __device__ __forceinline__ double rsqrt_pivot(double v) {
 //   3. the rows below take the rank-8 update; warp 0 updates only the next pivot block and goes on to its
 //      elimination, a chain of dependent operations, while the other warps update the rest.
 // One CTA; bound by the FP64 pipe of one SM (87 k FMAs at two per clock, about 21 us) and what is left of the
-// chain: 62 us.  Eliminating column by column with all warps queued the chain's operations behind the updates
-// in that pipe (80-90 us); separate factorisation and inversion kernels took 93 and 145 us.
+// chain: 56 us (62 with the other warps spread over all four schedulers).  Eliminating column by column with all
+// warps queued the chain's operations behind the updates in that pipe (80-90 us); separate factorisation and
+// inversion kernels took 93 and 145 us.
 constexpr int PB = 8;
 __global__ void __launch_bounds__(256) k_chol_inv_block(const double *A, double *Y, int64_t n, int64_t k0, int kb,
                                                         int *bad) {
@@ -130,12 +126,13 @@ __global__ void __launch_bounds__(256) k_chol_inv_block(const double *A, double 
                 if (lane == 0) atomicOr(bad, 1);
                 d = 1.0;
             }
+            // (l raw) beside the reciprocal: one operation follows it
+            const double p0 = -l * (pc > j ? a0 : pc == j ? 1.0 : z0);
+            const double p1 = -l * (pc + 1 > j ? a1 : pc + 1 == j ? 1.0 : z1);
             const double inv = rcp_pivot(d);
-            const double v0 = (pc > j ? a0 : pc == j ? 1.0 : z0) * inv;
-            const double v1 = (pc + 1 > j ? a1 : pc + 1 == j ? 1.0 : z1) * inv;
             if (pr > j) {
-                m0 = fma(-l, v0, pc == j ? 0.0 : m0);
-                m1 = fma(-l, v1, pc + 1 == j ? 0.0 : m1);
+                m0 = fma(p0, inv, pc == j ? 0.0 : m0);
+                m1 = fma(p1, inv, pc + 1 == j ? 0.0 : m1);
             } else if (pr == j) {
                 mine = d;
                 if (pc == j) m0 = 1.0;
@@ -190,8 +187,9 @@ __global__ void __launch_bounds__(256) k_chol_inv_block(const double *A, double 
                     m1 = fma(-l, s_l[I + pc + 1][q], m1);
                 }
                 pivots(m0, m1);
-            } else {
-                for (int i = I + w - 1; i < NB; i += 7) {
+            } else if (w & 3) {
+                // the warps of the other three schedulers: what shares warp 0's would queue its chain behind them
+                for (int i = I + (w >> 2) * 3 + (w & 3) - 1; i < NB; i += 6) {
                     double l[PB];
 #pragma unroll
                     for (int q = 0; q < PB; ++q) l[q] = s_l[i][q];

@@ -40,7 +40,7 @@ constexpr int kCols = GN / (kThreads / 128);       // output columns of a thread
 constexpr int kTmemCols = 512;                     // kWeights * GN
 constexpr size_t kGemmSmem = 2 * size_t(kStage) + 1024;  // + alignment
 constexpr long long kSpin = 2000000000ll;          // wait limit in clock cycles (about 1 s)
-constexpr int kScanInside = 256;                   // K up to which a tile finds its own row scales
+constexpr int kScanInside = 128;                   // K up to which a tile finds its own row scales (12 us at 256)
 
 __device__ __forceinline__ uint32_t saddr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
