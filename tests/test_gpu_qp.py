@@ -98,6 +98,19 @@ def test_pgs_colouring_general_graph(ctx, oracle):
         np.testing.assert_array_equal(col, ocol)
 
 
+@pytest.mark.parametrize("shape", [(1, 1), (2500, 1), (1, 2500), (257, 129), (900, 700), "graph5001"])
+def test_pgs_colouring_dependency_chains(ctx, oracle, shape):
+    """The colouring polls its predecessors inside one launch: single rows, a chain through every row, grids below and
+    above the resident threads (311,296), and an unstructured graph, against the sequential first-fit result."""
+    A = P.laplacian_2d(*shape) if isinstance(shape, tuple) else P.random_spd_graph(int(shape[5:]), 4, 1)
+    s = U.ProjectedGaussSeidel(ctx)
+    s.update(U.SparseMatrix(ctx, A))
+    col, nc = s.colouring()
+    ocol, onc = oracle.colouring(oracle.Matrix(A))
+    assert nc == onc
+    np.testing.assert_array_equal(col, ocol)
+
+
 def test_pgs_multicolour_matches_oracle(ctx, oracle):
     A, b, lb, ub = obstacle(48, True)
     Am = oracle.Matrix(A)
