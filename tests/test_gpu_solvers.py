@@ -247,6 +247,22 @@ def test_cholesky_solver_block_sizes(ctx, shape):
     assert rel(x.numpy(), xr) <= 1e-12
 
 
+@pytest.mark.parametrize("dim,size,levels", [(2, 768, 6), (3, 96, 4)])
+def test_power_method_forms(ctx, oracle, dim, size, levels):
+    """Chebyshev eigen-bounds where the power method runs in one cluster (48^2), over all SMs with one and two rows per
+    thread and rows of 9 and 27 entries (96^2, 192^2, 384^2, 24^3, 48^3) and in separate kernels (768^2, 96^3), the
+    start vectors drawn from one sequence over all levels.  The estimate is a norm of n rounded sums: 1e-12."""
+    A = P.laplacian_2d(size) if dim == 2 else P.laplacian_3d(size)
+    Ps = P.hierarchy_2d(size, levels) if dim == 2 else P.hierarchy_3d(size, levels)
+    omg = oracle.Multigrid(oracle.Matrix(A), Ps, smoother="chebyshev")
+    mg = U.Multigrid(ctx, smoother="chebyshev")
+    mg.set_transfer_operators(Ps)
+    M = U.SparseMatrix(ctx, A)
+    mg.update(M)
+    for l in range(1, levels):
+        np.testing.assert_allclose(mg.eigs(l), omg.eigs(l), rtol=1e-12)
+
+
 @pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 191, 257, 385, 578])
 @pytest.mark.parametrize("spread", [0, 40])
 def test_cholesky_split_products(ctx, n, spread):

@@ -199,4 +199,29 @@ __device__ __forceinline__ double warp_sum_of(const double *sh, int n) {
     return s;
 }
 
+// Launches a resident kernel: as one cluster (of at most 16 CTAs), or cooperatively.
+template <class Args>
+inline void launch_resident(Context &c, void (*kernel)(Args), const Args &args, int ctas, int threads, size_t smem,
+                            bool cluster) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(ctas));
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at[1];
+    if (cluster) {
+        UGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(ctas);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    UGPU_CUDA(cudaLaunchKernelEx(&cfg, kernel, args));
+    c.launches++;
+}
+
 }  // namespace ugpu

@@ -17,6 +17,7 @@
 
 #include "abi_util.cuh"
 #include "device_util.cuh"
+#include "pm_resident.cuh"
 #include "solver.cuh"
 
 namespace ugpu {
@@ -249,6 +250,7 @@ struct Level {
 // power-method scratch of one level
 struct PmScratch {
     Buffer v, w, st, part, cnt;  // st: [0] dot, [1] lambda, [2] lambda_old; int done, int skip, int64 it
+    Buffer sums;                 // the resident form's exchange
 };
 
 struct Transfer {
@@ -261,12 +263,13 @@ struct Transfer {
 class Multigrid final : public Solver {
 public:
     ~Multigrid() override {
-        if (!pm_streams_.empty() || pm_fork_) cudaStreamSynchronize(ctx->stream);
+        // the context may be gone already: its stream is held
+        if (!pm_streams_.empty() || pm_fork_) cudaStreamSynchronize(stream_->s);
         for (auto st : pm_streams_) cudaStreamDestroy(st);
         if (pm_fork_) cudaEventDestroy(pm_fork_);
         if (pm_join_) cudaEventDestroy(pm_join_);
     }
-    explicit Multigrid(Context *c) : Solver(c, UGPU_SOLVER_MULTIGRID) {
+    explicit Multigrid(Context *c) : Solver(c, UGPU_SOLVER_MULTIGRID), stream_(c->stream_ref) {
         prm["pre_smoothing_steps"] = 3;   // utopia_MultiLevelBase.hpp:35-42
         prm["post_smoothing_steps"] = 3;
         prm["smoother"] = 1;              // 0 Jacobi, 1 Chebyshev3level, 2 PointJacobi
@@ -504,6 +507,7 @@ public:
     }
 
 private:
+    std::shared_ptr<StreamRef> stream_;
     std::vector<Transfer> transfers_;
     std::vector<Level> levels_;
     DenseCholesky coarse_;
@@ -602,8 +606,8 @@ private:
     // PowerMethod::get_max_eig / compute_max_eig (utopia_PowerMethod.hpp:95-146) in FP64 for every
     // smoothed level; Chebyshev3level::init_eigs scales the result (utopia_Chebyshev3level.hpp:118-121).
     // The start vectors are drawn from the rand() sequence in level order (as the reference's
-    // levels are updated one after the other); the levels' iterations are independent, so they
-    // run concurrently on one stream per level (each with its own reduction scratch), joined
+    // levels are updated one after the other).  Levels that fit run in one kernel each
+    // (pm_resident.cu); the others' iterations are independent, so they run concurrently on one stream per level (each with its own reduction scratch), joined
     // back into the context's stream before the estimates are read.
     void power_methods() {
         const int L = n_levels();
@@ -646,8 +650,34 @@ private:
                 UGPU_CUDA(cudaMemsetAsync(ps.cnt.ptr, 0, ps.cnt.bytes, main));
             }
         }
+        // the smaller levels one after the other on the main stream, all iterations in one kernel each; the larger
+        // ones' streams start after them
+        std::vector<uint32_t> first(L, 0);
+        for (int l = 1; l < L; ++l) {
+            first[l] = drawn;
+            drawn += uint32_t(levels_[l].n);
+        }
+        auto start_vector = [&](int l) {
+            const int64_t n = levels_[l].n;
+            if (!n) return;
+            const int64_t warps = (n + kRandChunk - 1) / kRandChunk;
+            k_pm_start<<<unsigned((warps + 3) / 4), 128, 0, ctx->stream>>>(rand, first[l], n, pm_[l].v.as<double>());
+            ctx->launches++;
+        };
+        std::vector<char> resident(L, 0);
+        for (int l = 1; l < L; ++l) {
+            const Level &lv = levels_[l];
+            if (!pm_resident_fits(*ctx, *lv.A64)) continue;
+            resident[l] = 1;
+            PmScratch &ps = pm_[l];
+            start_vector(l);
+            ps.sums.ensure(pm_resident_bytes(*ctx));
+            pm_resident(*ctx, *lv.A64, ps.v.as<double>(), ps.w.as<double>(), ps.sums.ptr, ps.st.as<double>() + 1, tol,
+                        max_it);
+        }
         UGPU_CUDA(cudaEventRecord(pm_fork_, main));
         for (int l = 1; l < L; ++l) {
+            if (resident[l]) continue;
             const Level &lv = levels_[l];
             const int64_t n = lv.n;
             PmScratch &ps = pm_[l];
@@ -659,12 +689,7 @@ private:
             long long *itp = reinterpret_cast<long long *>(done + 2);
             const double *v = ps.v.as<double>(), *w = ps.w.as<double>();
             UGPU_CUDA(cudaMemsetAsync(ps.st.ptr, 0, ps.st.bytes, ctx->stream));
-            if (n) {
-                const int64_t warps = (n + kRandChunk - 1) / kRandChunk;
-                k_pm_start<<<unsigned((warps + 3) / 4), 128, 0, ctx->stream>>>(rand, drawn, n, ps.v.as<double>());
-                ctx->launches++;
-                drawn += uint32_t(n);
-            }
+            start_vector(l);
             DotArgs d{};
             d.nd = 1;
             d.dtype_a[0] = d.dtype_b[0] = UGPU_F64;
@@ -700,10 +725,11 @@ private:
         for (int l = 1; l < L; ++l) {
             UGPU_CUDA(cudaMemcpyAsync(&hs[size_t(l) * 3], pm_[l].st.ptr, 3 * sizeof(double), cudaMemcpyDeviceToHost,
                                       main));
-            UGPU_CUDA(cudaMemcpyAsync(&hd[size_t(l)], pm_[l].st.as<double>() + 3, sizeof(int), cudaMemcpyDeviceToHost,
-                                      main));
+            if (!resident[l])
+                UGPU_CUDA(cudaMemcpyAsync(&hd[size_t(l)], pm_[l].st.as<double>() + 3, sizeof(int),
+                                          cudaMemcpyDeviceToHost, main));
         }
-        UGPU_CUDA(cudaStreamSynchronize(main));
+        ctx->check_kernel_flags();
         for (int l = 1; l < L; ++l) {
             UGPU_CHECK(hd[size_t(l)] == 1, UGPU_ERR_INTERNAL, "power method: the stop test never held");
             Level &lv = levels_[l];

@@ -605,25 +605,7 @@ void MprgpResident::run(Context &c, const Mat &A, const double *b, double *x, co
                            : rpt == 1 ? (reg ? k_mprgp_resident<1, true, false> : k_mprgp_resident<1, false, false>)
                            : rpt == 2 ? (reg ? k_mprgp_resident<2, true, false> : k_mprgp_resident<2, false, false>)
                                       : k_mprgp_resident<4, false, false>;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(G));
-    cfg.blockDim = dim3(unsigned(nt));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = c.stream;
-    cudaLaunchAttribute at[1];
-    if (cl) {
-        UGPU_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = unsigned(G);
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    } else {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    UGPU_CUDA(cudaLaunchKernelEx(&cfg, f, a));
-    c.launches++;
+    launch_resident(c, f, a, int(G), nt, smem, cl);
 }
 
 }  // namespace ugpu
