@@ -83,23 +83,26 @@ struct RandTable {
 // out_i = rand_{first + i} / RAND_MAX + 1, i < n
 __global__ void __launch_bounds__(128) k_pm_start(const __grid_constant__ RandTable t, uint32_t first, int64_t n,
                                                   double *out) {
-    __shared__ uint32_t s_a[4][kRandWords], s_c[4][2 * kRandWords];
+    __shared__ uint32_t s_a[4][kRandWords], s_b[4][kRandWords], s_c[4][2 * kRandWords];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t begin = (blockIdx.x * int64_t(4) + w) * kRandChunk;
     if (begin >= n) return;
-    uint32_t *a = s_a[w], *c = s_c[w];
+    uint32_t *a = s_a[w], *b = s_b[w], *c = s_c[w];
     const uint32_t m = first + uint32_t(begin);
     if (lane < kRandWords) a[lane] = lane == 0 ? 1u : 0u;
     __syncwarp();
     for (int k = 0; k < 32; ++k) {
         if (!(m >> k & 1u)) continue;
         // a = a z^(2^k): coefficients `lane` and `lane + 31` of the product, then degrees 60 .. 31 folded three at a time
+        if (lane < kRandWords) b[lane] = t.pow[k][lane];  // lanes read different parameters: once, not per product
+        __syncwarp();
         uint32_t p0 = 0, p1 = 0;
+#pragma unroll
         for (int i = 0; i < kRandWords; ++i) {
             const uint32_t x = a[i];
             const int j0 = lane - i, j1 = lane + kRandWords - i;
-            if (j0 >= 0 && lane < kRandWords) p0 += x * t.pow[k][j0];
-            if (j1 < kRandWords) p1 += x * t.pow[k][j1];
+            if (j0 >= 0 && lane < kRandWords) p0 += x * b[j0];
+            if (j1 < kRandWords) p1 += x * b[j1];
         }
         if (lane < kRandWords) {
             c[lane] = p0;
