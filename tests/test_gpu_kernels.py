@@ -508,3 +508,28 @@ def test_fp64_rate_measurement(ctx):
     print(f"FP64 DFMA {dfma / 1e12:.3f} TFLOP/s, DMMA m8n8k4 {dmma / 1e12:.3f} TFLOP/s")
     assert 0.2e12 < dfma < 5e12
     assert 0.2e12 < dmma < 5e12
+
+
+@pytest.mark.parametrize("ka", [1, 7, 8, 9, 31, 32, 33, 65])
+@pytest.mark.parametrize("kb,pool", [(1, 2000), (7, 8), (9, 4000), (31, 40), (33, 126), (33, 4000)])
+def test_spgemm_row_lengths_around_the_groups(ctx, ka, kb, pool):
+    """Rows of A and B one below, at and above the lane groups' widths, landing on few or many columns (all warp
+    tiers): whole-number values, so the product is exact."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(1000 * ka + kb)
+    m, n = 133, 300
+
+    def rows(nr, nc, k):
+        k = np.minimum(nc, k - np.arange(nr) % 3 % k)
+        c = np.concatenate([rng.choice(nc, q, replace=False) for q in k])
+        M = sp.csr_matrix((rng.integers(1, 9, c.size).astype(float), (np.repeat(np.arange(nr), k), c)), shape=(nr, nc))
+        M.sort_indices()
+        return M
+
+    A, B = rows(m, n, ka), rows(n, pool, kb)
+    C = (A @ B).tocsr()
+    C.sort_indices()
+    rp, ci, v = U.SparseMatrix(ctx, P.CSR.from_scipy(A)).matmul(U.SparseMatrix(ctx, P.CSR.from_scipy(B))).csr()
+    assert (rp == C.indptr).all() and (ci == C.indices).all()
+    np.testing.assert_array_equal(v, C.data)

@@ -178,10 +178,13 @@ constexpr int kCtaTable = 8192;       // slots per CTA (rows with upper bound <=
 constexpr int kCtaRowsUb = 4096;
 constexpr int kCtaThreads = 256;
 
-__device__ __forceinline__ uint32_t hash_col(int32_t c, int mask) { return (uint32_t(c) * 2654435761u) & mask; }
+// Fibonacci hashing: the product's top bits.  Its low bits keep a column's low bits, and a grid whose lines are a
+// power of two long puts a row's columns in a few slots, one behind the other (the numeric products of a 128^3
+// Galerkin set-up took 6.7 ms with the low bits, 3.7 with the top ones).
+__device__ __forceinline__ uint32_t hash_col(int32_t c, int mask) { return (uint32_t(c) * 2654435761u) >> __clz(mask); }
 
-// insert column c; concurrent inserters hold distinct columns.  Returns the slot.
-__device__ __forceinline__ int hash_insert(int32_t *keys, int mask, int32_t c, int *n_unique) {
+// insert column c; concurrent inserters hold distinct columns.  Returns the slot; new entries count in n_new.
+__device__ __forceinline__ int hash_insert(int32_t *keys, int mask, int32_t c, int &n_new) {
     volatile int32_t *vk = keys;
     uint32_t h = hash_col(c, mask);
     while (true) {
@@ -190,7 +193,7 @@ __device__ __forceinline__ int hash_insert(int32_t *keys, int mask, int32_t c, i
         if (k == -1) {
             int32_t old = atomicCAS(&keys[h], -1, c);
             if (old == -1) {
-                if (n_unique) atomicAdd(n_unique, 1);
+                ++n_new;
                 return int(h);
             }
             if (old == c) return int(h);
@@ -213,10 +216,58 @@ __device__ __forceinline__ int table_size(int64_t ub, int cap) {
     return t;
 }
 
+// The products of row i of A B in A-row order by a warp: f(column, a, b) on the lane that holds the
+// product, step() on all lanes after each A entry, false to stop.  Bound by the latency of three dependent loads
+// (entry, row bounds, row) per A entry, so the lanes load 32 entries and their bounds at once and hand them round,
+// and each B row's first 32 entries are loaded while the row before is added (mid tier of a 128^3 Galerkin set-up
+// 1.25 -> 0.96 ms).
+template <bool NUMERIC, class V, class F, class S>
+__device__ __forceinline__ void for_products(int64_t i, int tid, const int32_t *arp,
+                                             const int32_t *aci, const V *acv, const int32_t *brp,
+                                             const int32_t *bci, const V *bcv, F f, S step) {
+    const int32_t a1 = arp[i + 1];
+    for (int32_t ka = arp[i]; ka < a1; ka += 32) {
+        const int left = min(32, a1 - ka);
+        int32_t b0 = 0, b1 = 0;
+        double a = 0.0;
+        if (tid < left) {
+            const int32_t j = aci[ka + tid];
+            b0 = brp[j];
+            b1 = brp[j + 1];
+            if (NUMERIC) a = cvt<double>(acv[ka + tid]);
+        }
+        int32_t s = __shfl_sync(0xffffffffu, b0, 0), e = __shfl_sync(0xffffffffu, b1, 0), c = 0;
+        double v = 0.0;
+        if (s + tid < e) {
+            c = bci[s + tid];
+            if (NUMERIC) v = cvt<double>(bcv[s + tid]);
+        }
+        for (int t = 0; t < left; ++t) {
+            const int32_t ns = __shfl_sync(0xffffffffu, b0, (t + 1) % 32);
+            const int32_t ne = t + 1 < left ? __shfl_sync(0xffffffffu, b1, (t + 1) % 32) : ns;
+            int32_t nc = 0;
+            double nv = 0.0;
+            if (ns + tid < ne) {
+                nc = bci[ns + tid];
+                if (NUMERIC) nv = cvt<double>(bcv[ns + tid]);
+            }
+            const double at = NUMERIC ? __shfl_sync(0xffffffffu, a, t) : 0.0;
+            if (s + tid < e) f(c, at, v);
+            for (int32_t kb = s + tid + 32; kb < e; kb += 32) f(bci[kb], at, NUMERIC ? cvt<double>(bcv[kb]) : 0.0);
+            __syncwarp();  // every product of this entry lands before the next entry's
+            if (!step()) return;
+            s = ns;
+            e = ne;
+            c = nc;
+            v = nv;
+        }
+    }
+}
+
 // One output row with G cooperating threads.  NUMERIC = false: count unique columns;
 // true: accumulate values and write the row sorted by column.
-template <class V, bool NUMERIC, bool CTA>
-__device__ void row_product(int64_t i, int tid, int G, int TS, int32_t *keys, double *vals, int32_t *lkeys,
+template <class V, bool NUMERIC, bool CTA, int G>
+__device__ void row_product(int64_t i, int tid, int TS, int32_t *keys, double *vals, int32_t *lkeys,
                             double *lvals, int *s_count, const int32_t *arp, const int32_t *aci, const V *acv,
                             const int32_t *brp, const int32_t *bci, const V *bcv, int64_t *cnt_out,
                             const int32_t *crp, int32_t *cci, V *ccv, unsigned gmask = 0xffffffffu) {
@@ -225,41 +276,80 @@ __device__ void row_product(int64_t i, int tid, int G, int TS, int32_t *keys, do
         keys[s] = -1;
         if (NUMERIC) vals[s] = 0.0;
     }
-    if (tid == 0) *s_count = 0;
+    if (CTA && tid == 0) *s_count = 0;
     group_sync<CTA>(gmask);
-    for (int32_t ka = arp[i]; ka < arp[i + 1]; ++ka) {
-        const int32_t j = aci[ka];
-        const double a = NUMERIC ? cvt<double>(acv[ka]) : 0.0;
-        const int32_t b1 = brp[j + 1];
-        for (int32_t kb = brp[j] + tid; kb < b1; kb += G) {
-            const int slot = hash_insert(keys, mask, bci[kb], NUMERIC ? nullptr : s_count);
-            if (NUMERIC) vals[slot] = fma(a, cvt<double>(bcv[kb]), vals[slot]);
+    int n_new = 0;
+    auto product = [&](int32_t c, double a, double b) {
+        const int slot = hash_insert(keys, mask, c, n_new);
+        if (NUMERIC) vals[slot] = fma(a, b, vals[slot]);
+    };
+    if constexpr (G != 32) {  // a CTA, or a short row's eight lanes, whose other groups hide the loads
+        for (int32_t ka = arp[i]; ka < arp[i + 1]; ++ka) {
+            const int32_t j = aci[ka];
+            const double a = NUMERIC ? cvt<double>(acv[ka]) : 0.0;
+            const int32_t b1 = brp[j + 1];
+            for (int32_t kb = brp[j] + tid; kb < b1; kb += G) product(bci[kb], a, NUMERIC ? cvt<double>(bcv[kb]) : 0.0);
+            group_sync<CTA>(gmask);  // every product of this j lands before the next j
         }
-        group_sync<CTA>(gmask);  // every product of this j lands before the next j
+    } else {
+        for_products<NUMERIC>(i, tid, arp, aci, acv, brp, bci, bcv, product, [] { return true; });
     }
     if (!NUMERIC) {
-        if (tid == 0) cnt_out[i] = *s_count;
+        if constexpr (CTA) {
+            if (n_new) atomicAdd(s_count, n_new);
+            __syncthreads();
+            if (tid == 0) cnt_out[i] = *s_count;
+        } else {
+            const int c = __reduce_add_sync(gmask, n_new);
+            if (tid == 0) cnt_out[i] = c;
+        }
         group_sync<CTA>(gmask);
         return;
     }
     // compact the occupied slots, then place each entry at its rank (sorted by column)
-    for (int s = tid; s < TS; s += G) {
+    int u = 0;
+    for (int s = tid; s < TS; s += G) {  // TS is a multiple of a warp group's G
         const int32_t k = keys[s];
+        int p;
+        if constexpr (CTA) {
+            if (k < 0) continue;
+            p = atomicAdd(s_count, 1);
+        } else {
+            const unsigned m = __ballot_sync(gmask, k >= 0) & gmask;
+            p = u + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+            u += __popc(m);
+        }
         if (k >= 0) {
-            const int p = atomicAdd(s_count, 1);
             lkeys[p] = k;
             lvals[p] = vals[s];
         }
     }
     group_sync<CTA>(gmask);
-    const int u = *s_count;
+    if constexpr (CTA) u = *s_count;
+    const int u4 = (u + 3) & ~3;  // the buffers hold a multiple of four entries
+    if (tid < u4 - u) lkeys[u + tid] = INT_MAX;
+    group_sync<CTA>(gmask);
     const int32_t base = crp[i];
-    for (int e = tid; e < u; e += G) {
-        const int32_t k = lkeys[e];
-        int rank = 0;
-        for (int t = 0; t < u; ++t) rank += (lkeys[t] < k);
-        cci[base + rank] = k;
-        ccv[base + rank] = cvt<V>(lvals[e]);
+    // Q entries of a lane against four keys per shared load: one entry per pass over single keys took longer
+    // than the products of a row of a hundred
+    constexpr int Q = G < 32 ? 1 : 4;
+    for (int e0 = tid; e0 < u; e0 += Q * G) {
+        int32_t k[Q];
+        int rank[Q] = {};
+#pragma unroll
+        for (int q = 0; q < Q; ++q) k[q] = e0 + q * G < u ? lkeys[e0 + q * G] : -1;
+        for (int t = 0; t < u4; t += 4) {
+            const int4 o = *reinterpret_cast<const int4 *>(lkeys + t);
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                rank[q] += (o.x < k[q]) + (o.y < k[q]) + (o.z < k[q]) + (o.w < k[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (k[q] >= 0) {
+                cci[base + rank[q]] = k[q];
+                ccv[base + rank[q]] = cvt<V>(lvals[e0 + q * G]);
+            }
     }
     group_sync<CTA>(gmask);
 }
@@ -279,19 +369,17 @@ constexpr size_t tier_smem() {
 }
 
 template <class V, bool NUMERIC, int TABLE, int ROWS_UB, int WARPS, bool APPEND>
-__global__ void __launch_bounds__(WARPS * 32) k_spgemm_warp(int64_t m, int64_t lo, const int64_t *ub,
-                                                            const int32_t *arp, const int32_t *aci, const V *acv,
-                                                            const int32_t *brp, const int32_t *bci, const V *bcv,
-                                                            int64_t *cnt, const int32_t *crp, int32_t *cci, V *ccv,
-                                                            int *big_rows, int *n_big) {
-    extern __shared__ unsigned char smem[];
+__global__ void __launch_bounds__(WARPS * 32, TABLE <= 256 ? 6 : 1)
+    k_spgemm_warp(int64_t m, int64_t lo, const int64_t *ub, const int32_t *arp, const int32_t *aci, const V *acv,
+                  const int32_t *brp, const int32_t *bci, const V *bcv, int64_t *cnt, const int32_t *crp,
+                  int32_t *cci, V *ccv, int *big_rows, int *n_big) {
+    extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double *vals = reinterpret_cast<double *>(smem) + size_t(w) * TABLE;
     double *lvals = reinterpret_cast<double *>(smem) + size_t(WARPS) * TABLE + size_t(w) * ROWS_UB;
     int32_t *ibase = reinterpret_cast<int32_t *>(smem + sizeof(double) * (TABLE + ROWS_UB) * WARPS);
     int32_t *keys = ibase + size_t(w) * TABLE;
     int32_t *lkeys = ibase + size_t(WARPS) * TABLE + size_t(w) * ROWS_UB;
-    __shared__ int s_count[WARPS];
     const int64_t gw = int64_t(blockIdx.x) * WARPS + w;
     const int64_t nw = int64_t(gridDim.x) * WARPS;
     for (int64_t i = gw; i < m; i += nw) {
@@ -301,8 +389,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_spgemm_warp(int64_t m, int64_t l
             if (APPEND && !NUMERIC && lane == 0) big_rows[atomicAdd(n_big, 1)] = int(i);
             continue;
         }
-        row_product<V, NUMERIC, false>(i, lane, 32, table_size(u, TABLE), keys, vals, lkeys, lvals, &s_count[w],
-                                       arp, aci, acv, brp, bci, bcv, cnt, crp, cci, ccv);
+        // numeric: the row's length is known, and the table it takes is smaller
+        const int64_t entries = NUMERIC ? crp[i + 1] - crp[i] : u;
+        row_product<V, NUMERIC, false, 32>(i, lane, table_size(entries, TABLE), keys, vals, lkeys, lvals, nullptr,
+                                           arp, aci, acv, brp, bci, bcv, cnt, crp, cci, ccv);
     }
 }
 
@@ -318,7 +408,7 @@ __global__ void __launch_bounds__(kSubWarps * 32) k_spgemm_sub(int64_t m, const 
                                                              const int32_t *aci, const V *acv, const int32_t *brp,
                                                              const int32_t *bci, const V *bcv, int64_t *cnt,
                                                              const int32_t *crp, int32_t *cci, V *ccv) {
-    extern __shared__ unsigned char smem[];
+    extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NG = kSubWarps * kSubGroups;  // groups per CTA
     const int lane = threadIdx.x & 31;
     const int g = threadIdx.x / kSubLanes;  // group within the CTA
@@ -329,13 +419,12 @@ __global__ void __launch_bounds__(kSubWarps * 32) k_spgemm_sub(int64_t m, const 
     int32_t *ibase = reinterpret_cast<int32_t *>(smem + sizeof(double) * (kTier0Table + kTier0Ub) * NG);
     int32_t *keys = ibase + size_t(g) * kTier0Table;
     int32_t *lkeys = ibase + size_t(NG) * kTier0Table + size_t(g) * kTier0Ub;
-    __shared__ int s_count[NG];
     const int64_t ng = int64_t(gridDim.x) * NG;
     for (int64_t i = int64_t(blockIdx.x) * NG + g; i < m; i += ng) {
         const int64_t u = ub[i];
         if (u > kTier0Ub) continue;  // the group's lanes agree: one row per group
-        row_product<V, NUMERIC, false>(i, tid, kSubLanes, table_size(u, kTier0Table), keys, vals, lkeys, lvals,
-                                       &s_count[g], arp, aci, acv, brp, bci, bcv, cnt, crp, cci, ccv, gmask);
+        row_product<V, NUMERIC, false, kSubLanes>(i, tid, kTier0Table, keys, vals, lkeys, lvals, nullptr, arp, aci,
+                                                  acv, brp, bci, bcv, cnt, crp, cci, ccv, gmask);
     }
 }
 
@@ -349,7 +438,7 @@ constexpr int kMidTable = 256, kMidCap = 128, kMidWarps = 8;
 constexpr size_t kMidSmem = (sizeof(int32_t) + sizeof(double)) * size_t(kMidTable + kMidCap) * kMidWarps;
 
 // hash_insert with a bounded probe sequence: -1 when the table is full
-__device__ __forceinline__ int hash_insert_bounded(int32_t *keys, int mask, int32_t c, int *n_unique) {
+__device__ __forceinline__ int hash_insert_bounded(int32_t *keys, int mask, int32_t c, int &n_new) {
     volatile int32_t *vk = keys;
     uint32_t h = hash_col(c, mask);
     for (int p = 0; p <= mask; ++p) {
@@ -358,7 +447,7 @@ __device__ __forceinline__ int hash_insert_bounded(int32_t *keys, int mask, int3
         if (k == -1) {
             const int32_t old = atomicCAS(&keys[h], -1, c);
             if (old == -1) {
-                atomicAdd(n_unique, 1);
+                ++n_new;
                 return int(h);
             }
             if (old == c) return int(h);
@@ -369,33 +458,22 @@ __device__ __forceinline__ int hash_insert_bounded(int32_t *keys, int mask, int3
 }
 
 // distinct columns of row i of A B with one warp and a table of TS slots, or -1 past cap
-__device__ int row_count_capped(int64_t i, int lane, int TS, int cap, int32_t *keys, int *s_count, int *s_over,
-                                const int32_t *arp, const int32_t *aci, const int32_t *brp, const int32_t *bci) {
+__device__ int row_count_capped(int64_t i, int lane, int TS, int cap, int32_t *keys, const int32_t *arp,
+                                const int32_t *aci, const int32_t *brp, const int32_t *bci) {
     const int mask = TS - 1;
     for (int t = lane; t < TS; t += 32) keys[t] = -1;
-    if (lane == 0) {
-        *s_count = 0;
-        *s_over = 0;
-    }
     __syncwarp();
-    bool over = false;
-    for (int32_t ka = arp[i]; ka < arp[i + 1] && !over; ++ka) {
-        const int32_t j = aci[ka];
-        const int32_t b1 = brp[j + 1];
-        for (int32_t kb = brp[j] + lane; kb < b1; kb += 32) {
-            if (*reinterpret_cast<volatile int *>(s_count) > cap) break;
-            if (hash_insert_bounded(keys, mask, bci[kb], s_count) < 0) {
-                *s_over = 1;
-                break;
-            }
-        }
-        __syncwarp();
-        over = *reinterpret_cast<volatile int *>(s_count) > cap || *reinterpret_cast<volatile int *>(s_over) != 0;
-        __syncwarp();  // every lane reads before any lane inserts again: `over` is warp-uniform
-    }
-    const int c = *reinterpret_cast<volatile int *>(s_count);
-    __syncwarp();
-    return over ? -1 : c;
+    int n_new = 0, count = 0;
+    for_products<false, double>(
+        i, lane, arp, aci, nullptr, brp, bci, nullptr,
+        [&](int32_t c, double, double) {
+            if (n_new <= TS && hash_insert_bounded(keys, mask, c, n_new) < 0) n_new = 2 * TS;  // full: past any cap
+        },
+        [&] {
+            count = __reduce_add_sync(0xffffffffu, n_new);
+            return count <= cap;  // warp-uniform
+        });
+    return count <= cap ? count : -1;
 }
 
 // symbolic mid tier: rows with kTier1Ub < ub <= kWarpRowsUb counted at the small size; those past
@@ -405,7 +483,6 @@ __global__ void __launch_bounds__(kMidWarps * 32) k_spgemm_mid_sym(int64_t m, co
                                                                  const int32_t *bci, int64_t *cnt, int *over,
                                                                  int *n_over, int *big, int *n_big) {
     __shared__ int32_t s_keys[kMidWarps][kMidTable];
-    __shared__ int s_count[kMidWarps], s_over[kMidWarps];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t nw = int64_t(gridDim.x) * kMidWarps;
     for (int64_t i = int64_t(blockIdx.x) * kMidWarps + w; i < m; i += nw) {
@@ -415,8 +492,7 @@ __global__ void __launch_bounds__(kMidWarps * 32) k_spgemm_mid_sym(int64_t m, co
             if (lane == 0) big[atomicAdd(n_big, 1)] = int(i);
             continue;
         }
-        const int c = row_count_capped(i, lane, kMidTable, kMidCap, s_keys[w], &s_count[w], &s_over[w], arp, aci,
-                                       brp, bci);
+        const int c = row_count_capped(i, lane, kMidTable, kMidCap, s_keys[w], arp, aci, brp, bci);
         if (lane == 0) {
             if (c >= 0) cnt[i] = c;
             else over[atomicAdd(n_over, 1)] = int(i);
@@ -431,21 +507,20 @@ __global__ void __launch_bounds__(kMidWarps * 32) k_spgemm_mid_num(int64_t m, co
                                                                  const int32_t *brp, const int32_t *bci,
                                                                  const V *bcv, const int32_t *crp, int32_t *cci,
                                                                  V *ccv) {
-    extern __shared__ unsigned char smem[];
+    extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double *vals = reinterpret_cast<double *>(smem) + size_t(w) * kMidTable;
     double *lvals = reinterpret_cast<double *>(smem) + size_t(kMidWarps) * kMidTable + size_t(w) * kMidCap;
     int32_t *ibase = reinterpret_cast<int32_t *>(smem + sizeof(double) * (kMidTable + kMidCap) * kMidWarps);
     int32_t *keys = ibase + size_t(w) * kMidTable;
     int32_t *lkeys = ibase + size_t(kMidWarps) * kMidTable + size_t(w) * kMidCap;
-    __shared__ int s_count[kMidWarps];
     const int64_t nw = int64_t(gridDim.x) * kMidWarps;
     for (int64_t i = int64_t(blockIdx.x) * kMidWarps + w; i < m; i += nw) {
         const int64_t u = ub[i];
         const int nz = crp[i + 1] - crp[i];
         if (u <= kTier1Ub || u > kWarpRowsUb || nz > kMidCap) continue;
-        row_product<V, true, false>(i, lane, 32, table_size(nz, kMidTable), keys, vals, lkeys, lvals, &s_count[w],
-                                    arp, aci, acv, brp, bci, bcv, nullptr, crp, cci, ccv);
+        row_product<V, true, false, 32>(i, lane, table_size(nz, kMidTable), keys, vals, lkeys, lvals, nullptr, arp,
+                                        aci, acv, brp, bci, bcv, nullptr, crp, cci, ccv);
     }
 }
 
@@ -457,19 +532,18 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_spgemm_warp_list(const in
                                                                        const int32_t *bci, const V *bcv,
                                                                        int64_t *cnt, const int32_t *crp,
                                                                        int32_t *cci, V *ccv) {
-    extern __shared__ unsigned char smem[];
+    extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double *vals = reinterpret_cast<double *>(smem) + size_t(w) * kWarpTable;
     double *lvals = reinterpret_cast<double *>(smem) + size_t(kWarpsPerCta) * kWarpTable + size_t(w) * kWarpRowsUb;
     int32_t *ibase = reinterpret_cast<int32_t *>(smem + sizeof(double) * (kWarpTable + kWarpRowsUb) * kWarpsPerCta);
     int32_t *keys = ibase + size_t(w) * kWarpTable;
     int32_t *lkeys = ibase + size_t(kWarpsPerCta) * kWarpTable + size_t(w) * kWarpRowsUb;
-    __shared__ int s_count[kWarpsPerCta];
     const int nw = gridDim.x * kWarpsPerCta;
     for (int b = blockIdx.x * kWarpsPerCta + w; b < nrows; b += nw) {
         const int64_t i = rows[b];
-        row_product<V, NUMERIC, false>(i, lane, 32, table_size(ub[i], kWarpTable), keys, vals, lkeys, lvals,
-                                       &s_count[w], arp, aci, acv, brp, bci, bcv, cnt, crp, cci, ccv);
+        row_product<V, NUMERIC, false, 32>(i, lane, table_size(ub[i], kWarpTable), keys, vals, lkeys, lvals,
+                                           nullptr, arp, aci, acv, brp, bci, bcv, cnt, crp, cci, ccv);
     }
 }
 
@@ -478,7 +552,7 @@ __global__ void __launch_bounds__(kCtaThreads) k_spgemm_cta(const int *big_rows,
                                                             const int32_t *arp, const int32_t *aci, const V *acv,
                                                             const int32_t *brp, const int32_t *bci, const V *bcv,
                                                             int64_t *cnt, const int32_t *crp, int32_t *cci, V *ccv) {
-    extern __shared__ unsigned char smem[];
+    extern __shared__ __align__(16) unsigned char smem[];
     double *vals = reinterpret_cast<double *>(smem);
     double *lvals = vals + kCtaTable;
     int32_t *keys = reinterpret_cast<int32_t *>(lvals + kCtaRowsUb);
@@ -487,8 +561,8 @@ __global__ void __launch_bounds__(kCtaThreads) k_spgemm_cta(const int *big_rows,
     for (int b = blockIdx.x; b < n_big; b += gridDim.x) {
         const int64_t i = big_rows[b];
         if (ub[i] > kCtaRowsUb) continue;  // wide row: k_spgemm_wide
-        row_product<V, NUMERIC, true>(i, threadIdx.x, blockDim.x, table_size(ub[i], kCtaTable), keys, vals, lkeys,
-                                      lvals, &s_count, arp, aci, acv, brp, bci, bcv, cnt, crp, cci, ccv);
+        row_product<V, NUMERIC, true, kCtaThreads>(i, threadIdx.x, table_size(ub[i], kCtaTable), keys, vals, lkeys,
+                                                   lvals, &s_count, arp, aci, acv, brp, bci, bcv, cnt, crp, cci, ccv);
     }
 }
 
@@ -508,7 +582,7 @@ __global__ void __launch_bounds__(kWideThreads) k_spgemm_wide(const int *big_row
                                                               const double *acv, const int32_t *brp,
                                                               const int32_t *bci, const double *bcv, int64_t *cnt,
                                                               const int32_t *crp, int32_t *cci, double *ccv) {
-    extern __shared__ unsigned char smem[];
+    extern __shared__ __align__(16) unsigned char smem[];
     double *acc = reinterpret_cast<double *>(smem);
     int *flag = reinterpret_cast<int *>(acc + kWideWindow);
     __shared__ int s_min, s_max, s_base, s_warp[kWideThreads / 32];
