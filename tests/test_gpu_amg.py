@@ -83,3 +83,64 @@ def test_amg_pcg_matches_oracle(ctx, oracle, name):
     xg = x.numpy()
     assert np.linalg.norm(b - A.matvec(xg)) <= atol * 1.0001
     assert np.linalg.norm(xg - xr) <= 1e-8 * np.linalg.norm(xr)
+
+
+def _stencil(nx, ny, nz, offsets, seed):
+    """A symmetric pattern with independent values of very different size in both directions, ordered by index."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(seed)
+    n = nx * ny * nz
+    i = np.arange(n)
+    x, y, z = i % nx, i // nx % ny, i // (nx * ny)
+    r, c = [i], [i]
+    for dx, dy, dz in offsets:
+        ok = ((x + dx >= 0) & (x + dx < nx) & (y + dy >= 0) & (y + dy < ny) & (z + dz >= 0) & (z + dz < nz))
+        r.append(i[ok])
+        c.append((i + dx + nx * (dy + ny * dz))[ok])
+    r, c = np.concatenate(r), np.concatenate(c)
+    A = sp.csr_matrix((rng.lognormal(0, 1.5, r.size) * rng.choice([-1.0, 1.0], r.size), (r, c)), shape=(n, n))
+    A.sort_indices()
+    return A
+
+
+_BOX = [(a, b, c) for a in (-1, 0, 1) for b in (-1, 0, 1) for c in (-1, 0, 1) if (a, b, c) != (0, 0, 0)]
+_STAR = [o for o in _BOX if sum(map(abs, o)) == 1]
+_WIDE = [(a, b, 0) for a in range(-3, 4) for b in range(-3, 4) if (a, b) != (0, 0)]
+AGGREGATE_FORMS = {
+    "star": (lambda: _stencil(27, 26, 25, _STAR, 1), {}),
+    "star_bmax1": (lambda: _stencil(27, 26, 25, _STAR, 2), dict(bmax=1, weight=0.9)),
+    "box": (lambda: _stencil(27, 26, 25, _BOX, 3), dict(bmax=9)),
+    "wide": (lambda: _stencil(135, 131, 1, _WIDE, 4), dict(weight=0.6)),
+    "wide_rows_of_a_strip": (lambda: _stencil(9000, 2, 1, _WIDE, 5), {}),
+    "few_rows_at_a_time": (lambda: _stencil(18000, 1, 1, [(-1, 0, 0), (1, 0, 0)], 6), {}),
+    "threshold": (lambda: _stencil(128, 128, 1, [o for o in _BOX if o[2] == 0], 7), {}),
+}
+
+
+@pytest.mark.parametrize("excluded", [False, True])
+@pytest.mark.parametrize("additive", [0, 1])
+@pytest.mark.parametrize("name", list(AGGREGATE_FORMS))
+def test_aggregates_of_large_levels(ctx, oracle, name, additive, excluded):
+    """The aggregation in dependency order is the sequential one: every row's aggregate, over stencils that take
+    one, four and eight lanes a row, rows with only a diagonal (their columns stay in other rows) and chains."""
+    make, kw = AGGREGATE_FORMS[name]
+    A = make()
+    if excluded:  # every 11th row keeps its diagonal only
+        import scipy.sparse as sp
+
+        keep = np.repeat(np.arange(A.shape[0]), np.diff(A.indptr))
+        ok = (keep % 11 != 3) | (A.indices == keep)
+        A = sp.csr_matrix((A.data[ok], (keep[ok], A.indices[ok])), shape=A.shape)
+        A.sort_indices()
+    Ac = P.CSR.from_scipy(A)
+    okw = dict(kw, use_additive_correction=additive)
+    ref, Pm = oracle.agglomerate(oracle.Matrix(Ac), **okw)
+    amg = U.AlgebraicMultigrid(ctx, smoother="jacobi", n_levels=2, **okw)
+    try:
+        amg.update(U.SparseMatrix(ctx, Ac))
+    except U.UgpuError as e:  # the values make no definite operator; the aggregates are there before its factor
+        assert "coarse operator is not symmetric positive definite" in str(e)
+    got, nc = amg.parent(0)
+    assert nc == Pm.ncols
+    np.testing.assert_array_equal(got, ref)
