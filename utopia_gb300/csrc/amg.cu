@@ -498,7 +498,7 @@ public:
         UGPU_CHECK(want_levels == 0 || want_levels >= 2, UGPU_ERR_ARG, "n_levels must be 0 (automatic) or >= 2");
         transfers_.clear();
         parents_.clear();
-        std::unique_ptr<Mat> owned;
+        std::vector<std::unique_ptr<Mat>> products;
         const Mat *cur = A;
         std::vector<int32_t> rp, ci, parent;
         std::vector<double> v, amax;
@@ -527,14 +527,15 @@ public:
             parents_.push_back(std::move(g.parent));
             auto next = ptap(*cur, *P);  // IPRTransfer::restrict(M): P^T M P
             transfers_.push_back(std::move(P));
-            owned = std::move(next);
-            cur = owned.get();
+            cur = next.get();
+            products.push_back(std::move(next));
         }
         UGPU_CHECK(!transfers_.empty(), UGPU_ERR_ARG, "algebraic multigrid: no coarse level");
         // Multigrid takes interpolation operators ordered coarse -> fine
         std::vector<const Mat *> P;
         for (auto it = transfers_.rbegin(); it != transfers_.rend(); ++it) P.push_back(it->get());
         mg_set_transfers(mg_.get(), P);
+        mg_set_products(mg_.get(), std::move(products));  // a second time they took 2.2 ms of kernels at 95 x 89 x 97
         mg_->update(A);
     }
 

@@ -301,8 +301,11 @@ public:
             t.R64 = transpose(*t.P64);          // IPRTransfer: R = transpose(I)
             transfers_.push_back(std::move(t));
         }
+        products_.clear();
         ready_ = false;
     }
+    // the Galerkin products of the operator of the next update, finest first, where the caller has them already
+    void set_products(std::vector<std::unique_ptr<Mat>> products) { products_ = std::move(products); }
 
     int n_levels() const { return int(levels_.size()); }
     const Level &level(int l) const { return levels_.at(l); }
@@ -312,6 +315,8 @@ public:
         UGPU_CHECK(A && A->nrows == A->ncols, UGPU_ERR_ARG, "multigrid: square operator required");
         UGPU_CHECK(A->vdtype == UGPU_F64, UGPU_ERR_ARG, "multigrid: FP64 fine operator required");
         UGPU_CHECK(!transfers_.empty(), UGPU_ERR_STATE, "Provide interpolation operators first");
+        auto products = std::move(products_);
+        products_.clear();
         op = A;
         vdt_ = (int(get("precision")) == UGPU_F64) ? UGPU_F64 : UGPU_F32;
         const int sdt = int(get("precision"));
@@ -345,6 +350,8 @@ public:
                     std::shared_ptr<PtapPlan> plan;
                     lev[i].A64own = ptap_with_plan(*lev[i - 1].A64, *t.P64, plan);
                     lev[i].A64own->ptap_plan = std::move(plan);
+                } else if (int(products.size()) == L - 1) {
+                    lev[i].A64own = std::move(products[size_t(i - 1)]);
                 } else {
                     lev[i].A64own = ptap(*lev[i - 1].A64, *t.P64);
                 }
@@ -512,6 +519,7 @@ public:
 private:
     std::shared_ptr<StreamRef> stream_;
     std::vector<Transfer> transfers_;
+    std::vector<std::unique_ptr<Mat>> products_;
     std::vector<Level> levels_;
     DenseCholesky coarse_;
     int vdt_ = UGPU_F64;
@@ -958,6 +966,12 @@ void mg_set_transfers(Solver *s, const std::vector<const Mat *> &P) {
     auto m = dynamic_cast<Multigrid *>(s);
     UGPU_CHECK(m, UGPU_ERR_ARG, "not a multigrid solver");
     m->set_transfers(P);
+}
+
+void mg_set_products(Solver *s, std::vector<std::unique_ptr<Mat>> products) {
+    auto m = dynamic_cast<Multigrid *>(s);
+    UGPU_CHECK(m, UGPU_ERR_ARG, "not a multigrid solver");
+    m->set_products(std::move(products));
 }
 
 }  // namespace ugpu

@@ -146,6 +146,7 @@ int mg_n_levels(const Solver *s);
 std::unique_ptr<Mat> mg_level_matrix(const Solver *s, int l);
 void mg_eigs(const Solver *s, int l, double *emax, double *emin);
 void mg_set_transfers(Solver *s, const std::vector<const Mat *> &P);
+void mg_set_products(Solver *s, std::vector<std::unique_ptr<Mat>> products);
 // LinearMultiLevel::fix_semidefinite_operator: diagonal entries with |a_ii| < 1e-12 get +1
 void fix_semidefinite_operator(Context &ctx, Mat &J);
 // the monotone multigrid's counterparts (false / -1 / null: s is not a monotone multigrid)
