@@ -282,6 +282,20 @@ def test_cholesky_split_products(ctx, n, spread):
     assert rel(d * x.numpy(), y) <= 1e-12
 
 
+@pytest.mark.parametrize("n", [511, 512, 513, 639, 641, 769, 1025])
+def test_cholesky_products_around_the_fp64_tiles(ctx, n):
+    """Halves of 256 rows and less go through the FP64 tiles, longer ones through the split products: sizes on both
+    sides, ragged against the tiles of both (8, 64, 128).  n eps cond bounds the error: 1025 * 2.2e-16 * 5 = 1.2e-12."""
+    import scipy.sparse as sp
+    rng = np.random.default_rng(n)
+    M = rng.standard_normal((n, n))
+    B = M @ M.T / n + np.eye(n)
+    y = rng.standard_normal(n)
+    x = U.Vector(ctx, n=n)
+    U.CholeskySolver(ctx).solve(U.SparseMatrix(ctx, P.CSR.from_scipy(sp.csr_matrix(B))), U.Vector(ctx, B @ y), x)
+    assert rel(x.numpy(), y) <= 1.2e-12
+
+
 def test_cholesky_solver_factored_inverse_above_4096(ctx):
     """Coarse sizes above 4096 keep the inverse factored (Y = L^-1 and Y^T in one buffer, two
     triangular GEMVs per solve): FP64 and FP32 vectors against a direct solve."""

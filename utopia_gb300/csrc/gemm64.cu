@@ -421,6 +421,55 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm64(const Gemm64 g, const ui
     }
 }
 
+// Small products on the FP64 pipes of the whole chip: a CTA takes 8 x 8 outputs, four threads an output with
+// every fourth k each.  One or two CTAs of k_gemm64 are bound by their own splitting and rounding (18 us at 64^3,
+// 28 at 128^3, 37 at 256^3, on 1, 2 and 8 SMs); these FMAs are 0.9 k, 6.9 k and 55 k clocks of all the pipes, where
+// the two forms meet.  Factor and inverse of 4096 rows: 14.5 ms with none of the products here, 12.6 up to 64^3,
+// 11.2 up to 128^3, 10.6 up to 256^3.
+constexpr int kSmallK = 256;
+constexpr int64_t kSmallWork = 1 << 24;
+constexpr int kSmallTile = 8, kSmallRow = kSmallK + 4;  // a row's pad puts the lanes of a half-warp on all banks
+__global__ void __launch_bounds__(256) k_gemm64_small(const Gemm64 g) {
+    const int m0 = blockIdx.y * kSmallTile, n0 = blockIdx.x * kSmallTile;
+    if ((g.flags & kGemmLower) && n0 > m0 + kSmallTile - 1) return;
+    __shared__ double s[2][kSmallTile][kSmallRow];
+    int k0 = 0, k1 = g.K;
+    if (g.flags & kGemmKFromN) k0 = max(k0, n0);
+    if (g.flags & kGemmKFromM) k0 = max(k0, m0);
+    if (g.flags & kGemmKToN) k1 = min(k1, n0 + kSmallTile);
+    if (g.flags & kGemmKToM) k1 = min(k1, m0 + kSmallTile);
+    const int len = k1 - k0, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    double v[2][kSmallK / 32];
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const int64_t rs = o ? g.b_row : g.a_row, ks = o ? g.b_k : g.a_k;
+        const int r = ks == 1 ? warp : t & 7, kk = ks == 1 ? lane : t >> 3;
+        const int rows = o ? g.N - n0 : g.M - m0;
+        const double *p = (o ? g.B + n0 * rs : g.A + m0 * rs) + r * rs + int64_t(k0 + kk) * ks;
+#pragma unroll
+        for (int q = 0; q < kSmallK / 32; ++q) v[o][q] = (r < rows && kk + 32 * q < len) ? __ldg(p + 32 * q * ks) : 0.0;
+    }
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const bool along = (o ? g.b_k : g.a_k) == 1;
+        const int r = along ? warp : t & 7, kk = along ? lane : t >> 3;
+#pragma unroll
+        for (int q = 0; q < kSmallK / 32; ++q)
+            if (32 * q < len) s[o][r][kk + 32 * q] = v[o][q];
+    }
+    __syncthreads();
+    const int j = lane >> 2;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int k = lane & 3; k < len; k += 4) acc = fma(s[0][warp][k], s[1][j][k], acc);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    if ((lane & 3) || m0 + warp >= g.M || n0 + j >= g.N) return;
+    if (g.negate) acc = -acc;
+    double *C = g.C + int64_t(m0 + warp) * g.ldc + n0 + j;
+    *C = g.add ? *C + acc : acc;
+}
+
 }  // namespace
 
 void gemm64(Context &c, const Gemm64 &args, Buffer &scales) {
@@ -433,6 +482,13 @@ void gemm64(Context &c, const Gemm64 &args, Buffer &scales) {
     UGPU_CHECK(g.K <= 16384, UGPU_ERR_UNSUPPORTED, "gemm64: K is limited to 16384");
     UGPU_CHECK((g.a_row == 1 || g.a_k == 1) && (g.b_row == 1 || g.b_k == 1), UGPU_ERR_INTERNAL,
                "gemm64: operand strides");
+    if (g.K <= kSmallK && int64_t(g.M) * g.N * g.K <= kSmallWork) {
+        const dim3 tiles(unsigned((g.N + kSmallTile - 1) / kSmallTile), unsigned((g.M + kSmallTile - 1) / kSmallTile));
+        k_gemm64_small<<<tiles, 256, 0, c.stream>>>(g);
+        c.launches++;
+        UGPU_LAUNCH_CHECK();
+        return;
+    }
     uint32_t *eA = nullptr, *eB = nullptr;
     if (g.K > kScanInside) {
         scales.ensure(sizeof(uint32_t) * (size_t(g.M) + size_t(g.N)));
