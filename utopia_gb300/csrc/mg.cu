@@ -56,9 +56,9 @@ struct GlibcRand {
 // warp jumps to its own position m (a product of the tabulated powers z^(2^k)) and goes on from there 31
 // words at a time: word i of the next window is a sum of every third word of this one.  The values are those of
 // the sequential generator, which took 9 ms on the host for the 2.4 million rows of a 128^3 hierarchy, with
-// the copy to the device; this takes 0.26 ms.
+// the copy to the device; this takes 0.075 ms.
 constexpr int kRandWords = 31;
-constexpr int kRandChunk = 64 * kRandWords;  // words per warp: the jump costs as much as about 100 windows
+constexpr int kRandChunk = 16 * kRandWords;  // words per warp
 struct RandTable {
     uint32_t base[2 * kRandWords - 1];   // x_0 .. x_60
     uint32_t pow[32][kRandWords];        // z^(2^k)
@@ -80,51 +80,68 @@ struct RandTable {
     }
 };
 
-// out_i = rand_{first + i} / RAND_MAX + 1, i < n
-__global__ void __launch_bounds__(128) k_pm_start(const __grid_constant__ RandTable t, uint32_t first, int64_t n,
-                                                  double *out) {
-    __shared__ uint32_t s_a[4][kRandWords], s_b[4][kRandWords], s_c[4][2 * kRandWords];
+// the start vectors of several levels in one launch: out_i = rand_{first + i} / RAND_MAX + 1, i < n, from warp `warp`
+constexpr int kRandLevels = 16;
+struct RandLevels {
+    int count = 0;
+    int64_t warps = 0;
+    struct {
+        uint32_t first;
+        int64_t n, warp;
+        double *out;
+    } at[kRandLevels];
+};
+
+// Bound by the latency of a warp's jump, one product per set bit of its position: its coefficients stay in registers,
+// the factor in shared memory with zeros at both ends.  512 x 512 hierarchy: all levels 18 us, with a launch per
+// level and the folding of degrees 60 .. 31 in ten steps through shared memory 38 us each.
+__global__ void __launch_bounds__(128) k_pm_start(const __grid_constant__ RandTable t,
+                                                  const __grid_constant__ RandLevels levels) {
+    __shared__ uint32_t s_b[4][3 * kRandWords];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t begin = (blockIdx.x * int64_t(4) + w) * kRandChunk;
-    if (begin >= n) return;
-    uint32_t *a = s_a[w], *b = s_b[w], *c = s_c[w];
-    const uint32_t m = first + uint32_t(begin);
-    if (lane < kRandWords) a[lane] = lane == 0 ? 1u : 0u;
-    __syncwarp();
+    const int64_t warp = blockIdx.x * int64_t(4) + w;
+    if (warp >= levels.warps) return;
+    int l = 0;
+    while (l + 1 < levels.count && levels.at[l + 1].warp <= warp) ++l;
+    const int64_t begin = (warp - levels.at[l].warp) * kRandChunk, end = min(levels.at[l].n, begin + kRandChunk);
+    double *out = levels.at[l].out;
+    const uint32_t m = levels.at[l].first + uint32_t(begin);
+    uint32_t *b = s_b[w];
+    if (lane < kRandWords) b[lane] = b[lane + 2 * kRandWords] = 0;
+    uint32_t a = lane == 0 ? 1u : 0u;  // coefficient `lane`
     for (int k = 0; k < 32; ++k) {
         if (!(m >> k & 1u)) continue;
-        // a = a z^(2^k): coefficients `lane` and `lane + 31` of the product, then degrees 60 .. 31 folded three at a time
-        if (lane < kRandWords) b[lane] = t.pow[k][lane];  // lanes read different parameters: once, not per product
+        // a = a z^(2^k): coefficients `lane` and `lane + 31` of the product
+        __syncwarp();
+        if (lane < kRandWords) b[lane + kRandWords] = t.pow[k][lane];
         __syncwarp();
         uint32_t p0 = 0, p1 = 0;
 #pragma unroll
         for (int i = 0; i < kRandWords; ++i) {
-            const uint32_t x = a[i];
-            const int j0 = lane - i, j1 = lane + kRandWords - i;
-            if (j0 >= 0 && lane < kRandWords) p0 += x * b[j0];
-            if (j1 < kRandWords) p1 += x * b[j1];
+            const uint32_t x = __shfl_sync(0xffffffffu, a, i);
+            p0 += x * b[min(lane, kRandWords - 1) + kRandWords - i];
+            p1 += x * b[min(lane, kRandWords - 1) + 2 * kRandWords - i];
         }
-        if (lane < kRandWords) {
-            c[lane] = p0;
-            c[lane + kRandWords] = p1;
+        if (lane >= kRandWords) p0 = p1 = 0;
+        // degree d >= 31 goes to d - 3 and d - 31: the high half becomes its sums with stride 3 from above
+#pragma unroll
+        for (int o = 3; o < kRandWords; o *= 2) {
+            const uint32_t u = __shfl_down_sync(0xffffffffu, p1, o);
+            if (lane + o < kRandWords) p1 += u;
         }
-        __syncwarp();
-        for (int d = 2 * kRandWords - 2; d >= kRandWords; d -= 3) {
-            if (lane < 3) {
-                c[d - lane - 3] += c[d - lane];
-                c[d - lane - 31] += c[d - lane];
-            }
-            __syncwarp();
-        }
-        if (lane < kRandWords) a[lane] = c[lane];
-        __syncwarp();
+        const uint32_t low = __shfl_sync(0xffffffffu, p1, lane >= 28 ? lane - 28 : 0);
+        a = p0 + p1 + (lane >= 28 ? low : 0u);
     }
     uint32_t x = 0;
-    if (lane < kRandWords)
-        for (int j = 0; j < kRandWords; ++j) x += a[j] * t.base[lane + j];
-    const int64_t end = min(n, begin + kRandChunk);
-    for (int64_t i = begin; i < end; i += kRandWords) {
-        if (lane < kRandWords && i + lane < end) out[i + lane] = (double(int32_t(x >> 1)) / 2147483647.0) + 1;
+#pragma unroll
+    for (int j = 0; j < kRandWords; ++j) {
+        const uint32_t c = __shfl_sync(0xffffffffu, a, j);
+        if (lane < kRandWords) x += c * t.base[lane + j];
+    }
+#pragma unroll 4
+    for (int q = 0; q < kRandChunk / kRandWords; ++q) {
+        const int64_t i = begin + q * kRandWords + lane;
+        if (lane < kRandWords && i < end) out[i] = (double(int32_t(x >> 1)) / 2147483647.0) + 1;
         const uint32_t last = __shfl_sync(0xffffffffu, x, 28 + lane % 3);
         uint32_t s = x;
 #pragma unroll
@@ -668,20 +685,30 @@ private:
             first[l] = drawn;
             drawn += uint32_t(levels_[l].n);
         }
-        auto start_vector = [&](int l) {
-            const int64_t n = levels_[l].n;
-            if (!n) return;
-            const int64_t warps = (n + kRandChunk - 1) / kRandChunk;
-            k_pm_start<<<unsigned((warps + 3) / 4), 128, 0, ctx->stream>>>(rand, first[l], n, pm_[l].v.as<double>());
-            ctx->launches++;
+        RandLevels draw;
+        auto flush = [&] {
+            if (draw.warps) {
+                k_pm_start<<<unsigned((draw.warps + 3) / 4), 128, 0, main>>>(rand, draw);
+                ctx->launches++;
+            }
+            draw = RandLevels();
         };
+        for (int l = 1; l < L; ++l) {
+            auto &d = draw.at[draw.count++];
+            d.first = first[l];
+            d.n = levels_[l].n;
+            d.warp = draw.warps;
+            d.out = pm_[l].v.as<double>();
+            draw.warps += (d.n + kRandChunk - 1) / kRandChunk;
+            if (draw.count == kRandLevels) flush();
+        }
+        flush();
         std::vector<char> resident(L, 0);
         for (int l = 1; l < L; ++l) {
             const Level &lv = levels_[l];
             if (!pm_resident_fits(*ctx, *lv.A64)) continue;
             resident[l] = 1;
             PmScratch &ps = pm_[l];
-            start_vector(l);
             ps.sums.ensure(pm_resident_bytes(*ctx));
             pm_resident(*ctx, *lv.A64, ps.v.as<double>(), ps.w.as<double>(), ps.sums.ptr, ps.st.as<double>() + 1, tol,
                         max_it);
@@ -700,7 +727,6 @@ private:
             long long *itp = reinterpret_cast<long long *>(done + 2);
             const double *v = ps.v.as<double>(), *w = ps.w.as<double>();
             UGPU_CUDA(cudaMemsetAsync(ps.st.ptr, 0, ps.st.bytes, ctx->stream));
-            start_vector(l);
             DotArgs d{};
             d.nd = 1;
             d.dtype_a[0] = d.dtype_b[0] = UGPU_F64;
