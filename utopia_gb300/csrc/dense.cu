@@ -451,7 +451,8 @@ __global__ void __launch_bounds__(256) k_gemv64_warp(const double *M, int64_t n,
 // The same product for coarse levels whose right-hand side fits shared memory: r is converted to
 // FP64 once per CTA into shared memory, and each row is split over two warps (four rows per CTA),
 // so every lane has only a few independent 16-byte row loads and the grid keeps enough of them
-// in flight to stream the inverse at HBM rate.
+// in flight to stream the inverse.  Eight loads of a lane are in flight (r's and the rows'): 4096 rows 38 us, where
+// four took 49 and the FP64 pipes need 27.
 constexpr int kGemvSmemMax = 96 * 1024;  // bytes of r staged per CTA
 template <class VT>
 __global__ void __launch_bounds__(256) k_gemv64_split(const double *M, int64_t n, const VT *r, VT *x,
@@ -459,7 +460,8 @@ __global__ void __launch_bounds__(256) k_gemv64_split(const double *M, int64_t n
     extern __shared__ __align__(16) double sr[];  // r in FP64
     __shared__ double part[8];
     if (done && *done) return;
-    for (int64_t j = threadIdx.x; j < n; j += blockDim.x) sr[j] = cvt<double>(r[j]);
+#pragma unroll 8
+    for (int64_t j = threadIdx.x; j < n; j += 256) sr[j] = cvt<double>(__ldg(r + j));
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rl = warp >> 1, q = warp & 1;  // row of the four, half of the row
@@ -472,7 +474,7 @@ __global__ void __launch_bounds__(256) k_gemv64_split(const double *M, int64_t n
                 const int64_t n2 = n >> 1, c0 = q * n2 / 2, c1 = (q + 1) * n2 / 2;
                 const double2 *rv = reinterpret_cast<const double2 *>(row);
                 const double2 *xv = reinterpret_cast<const double2 *>(sr);
-#pragma unroll 4
+#pragma unroll 8
                 for (int64_t c = c0 + lane; c < c1; c += 32) {
                     const double2 a = __ldg(rv + c), b = xv[c];
                     s0 = fma(a.x, b.x, s0);
@@ -480,6 +482,7 @@ __global__ void __launch_bounds__(256) k_gemv64_split(const double *M, int64_t n
                 }
             } else {
                 const int64_t c0 = q * n / 2, c1 = (q + 1) * n / 2;
+#pragma unroll 8
                 for (int64_t c = c0 + lane; c < c1; c += 32) s0 = fma(__ldg(row + c), sr[c], s0);
             }
         }
