@@ -533,3 +533,37 @@ def test_spgemm_row_lengths_around_the_groups(ctx, ka, kb, pool):
     rp, ci, v = U.SparseMatrix(ctx, P.CSR.from_scipy(A)).matmul(U.SparseMatrix(ctx, P.CSR.from_scipy(B))).csr()
     assert (rp == C.indptr).all() and (ci == C.indices).all()
     np.testing.assert_array_equal(v, C.data)
+
+
+@pytest.mark.parametrize("kind", ["diagonals", "columns", "anchors"])
+@pytest.mark.parametrize("width", [10, 18, 19, 27])
+def test_sell_one_row_per_lane_has_the_same_bits(ctx, kind, width):
+    """Up to 131,072 rows (65,536 with explicit columns) a row of more than nine entries takes one lane, above that
+    two rows share one: a lower triangular matrix cut there and 63 rows later gives the same first rows, bit for
+    bit, in every kind of slice, and both are the FP64 product to width * 2^-52 of the row's magnitudes."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(width)
+    cut = 65536 if kind == "columns" else 131072
+    n = cut + 63
+    i = np.arange(n)
+    if kind == "diagonals":
+        c = i[:, None] - np.sort(rng.choice(4000, width, replace=False))
+    elif kind == "anchors":
+        c = (i // 5)[:, None] + np.sort(rng.choice(900, width, replace=False)) - 900
+    else:
+        c = i[:, None] - np.cumsum(rng.integers(1, 300, (n, width)), axis=1)
+    ok = (c >= 0) & (c <= i[:, None])
+    r = np.broadcast_to(i[:, None], c.shape)
+    A = sp.csr_matrix((rng.standard_normal(int(ok.sum())), (r[ok], c[ok])), shape=(n, n))
+    A.sort_indices()
+    x = rng.standard_normal(n)
+    got = []
+    for m in (cut, n):
+        B = A[:m, :m].tocsr()
+        y = U.Vector(ctx, n=m)
+        U.SparseMatrix(ctx, P.CSR.from_scipy(B)).apply(U.Vector(ctx, x[:m]), y)
+        got.append(y.numpy())
+        bound = width * 2.0 ** -52 * (abs(B) @ np.abs(x[:m]))
+        assert (np.abs(got[-1] - B @ x[:m]) <= bound).all()
+    np.testing.assert_array_equal(got[0], got[1][:cut])

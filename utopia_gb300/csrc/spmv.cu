@@ -780,6 +780,66 @@ __global__ void UGPU_SELL_BOUNDS k_sell_spmv(SellView m, EpiParams<T> e) {
     }
 }
 
+// The same product with one row per lane (FP64; a warp takes 32 of a slice's 64 rows), for matrices whose slices do
+// not fill the chip with warps: there the time is the chain of loads per warp.  All loads of kRowSlots slots are in
+// flight together, half as many rows per warp need half as many gathers, and twice as many warps run: a level of
+// 32,768 rows with 27 points took 15 to 17 us in a V-cycle, a V-cycle CG iteration on 128^3 0.78 ms and takes 0.72.
+// A row's products add in the same order as above: the same bits.
+constexpr int kRowSlots = 9;  // a 27-point row in three rounds, a 7- or 9-point row in one
+template <int EPI>
+__global__ void __launch_bounds__(kSpmvWarps * 32, 3) k_sell_rows(SellView m, EpiParams<double> e) {
+    if ((e.done && *e.done) || (e.gate && !*e.gate)) return;
+    constexpr int R = 2, S = 32 * R;
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    const int cmax = int(m.ncols) - 1;
+    for (int64_t hs = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; hs < R * m.nslices; hs += nwarps) {
+        const int64_t s = hs / R;
+        const int p = int(hs % R) * 32 + lane;  // the row's position in the slice
+        const int row = int(s * S) + (m.il ? p / R + 32 * (p % R) : p);
+        const int4 q = __ldg(m.hdr + s);
+        const int tag = q.z, aux = q.w;
+        const double *vals = static_cast<const double *>(m.vals) + ((int64_t(uint32_t(q.y)) << 32) | uint32_t(q.x)) + p;
+        const int w = tag < 0 ? -tag : tag >= kAnchoredTag ? tag - kAnchoredTag : tag;
+        const int32_t *cols = m.cols + aux + p;
+        int first = row;  // gathers at first + key, or at explicit columns
+        const int32_t *keys = m.offs + aux;
+        if (tag >= kAnchoredTag) {
+            first = __ldg(cols);
+            keys = m.cols + aux + S;
+        }
+        double acc = 0.0;
+        for (int k0 = 0; k0 < w; k0 += kRowSlots) {
+            double v[kRowSlots], x[kRowSlots];
+            int c[kRowSlots];
+#pragma unroll
+            for (int k = 0; k < kRowSlots; ++k) {
+                v[k] = 0.0;
+                c[k] = 0;
+                if (k0 + k < w) {
+                    v[k] = __ldcs(vals + int64_t(k0 + k) * S);
+                    c[k] = tag < 0 ? __ldcs(cols + int64_t(k0 + k) * S) : __ldg(keys + k0 + k);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kRowSlots; ++k) {
+                if (tag >= 0) c[k] = min(max(first + c[k], 0), cmax);
+                x[k] = k0 + k < w ? __ldg(e.x + c[k]) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kRowSlots; ++k)
+                if (k0 + k < w) acc = fma(v[k], x[k], acc);
+        }
+        if (row < m.nrows) {
+            double xr = 0.0;
+            if constexpr (epi_reads_x<EPI, 0, false>()) xr = __ldg(e.x + row);
+            const double out = epilogue<double, EPI>(e, row, acc, xr);
+            e.y[row] = out;
+            if constexpr (epi_writes_sw<EPI>()) e.sw_out[row] = e.sw[row] * out;
+        }
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // Shared-memory staged sliced-ELL product (FP32 vectors; FP32 or BF16 values; every slice
 // diagonal, lane-interleaved rows).
@@ -1392,12 +1452,27 @@ int spmv_grid(const Context &ctx, int64_t units_per_cta_work, int64_t total) {
     return int(g);
 }
 
+// Slices up to which k_sell_rows runs rows of more than kRowSlots entries.  Back to back, 27 points: 13,824 rows
+// 6.2 us against 8.5 in the register kernel, 32,768 6.2 / 9.8, 110,592 10.3 / 12.3, 262,144 22.6 / 20.5; 5 points
+// 65,536 rows 6.2 / 4.1, whose one round of loads the register kernel has in flight with fewer warps.  With explicit
+// columns half as many: 34,000 rows of an aggregation hierarchy 7.5 / 13.5, 65,000 rows 15 / 14.
+constexpr int64_t kRowSlices = 2048;
+
 template <class V, class T, int R, int EPI, int XM, bool DOT>
 void sell_launch(Context &ctx, const Mat &A, const SpmvArgs &a) {
     const Sell &s = *A.sell;
     SellView m{s.hdr.as<int4>(), s.slice_ptr.as<int64_t>(), s.slice_w.as<int32_t>(), s.slice_aux.as<int64_t>(),
                s.offs.as<int32_t>(),
                s.cols.as<int32_t>(), s.vals.ptr, s.nslices, A.nrows, A.ncols, s.interleaved ? 1 : 0};
+    if constexpr (std::is_same<V, double>::value && std::is_same<T, double>::value && XM == 0 && !DOT) {
+        const bool keyed = s.ndiag_slices + s.nanch_slices == s.nslices;
+        if (!a.fa && s.max_width > kRowSlots && s.nslices <= (keyed ? kRowSlices : kRowSlices / 2)) {
+            const int64_t ctas = (R * s.nslices + kSpmvWarps - 1) / kSpmvWarps;
+            const int g = int(std::max<int64_t>(1, std::min<int64_t>(ctas, int64_t(ctx.sms) * 16)));
+            k_sell_rows<EPI><<<g, kSpmvWarps * 32, 0, ctx.stream>>>(m, make_epi<T>(a));
+            return;
+        }
+    }
     // one wave of resident CTAs (grid-stride over slices)
     static int per_sm = 0;
     if (per_sm == 0) {
