@@ -331,9 +331,9 @@ __global__ void k_agg_prolongator(const unsigned long long *word, const int64_t 
 }
 
 struct Aggregates {
-    Buffer parent;              // aggregate of each row
+    std::vector<int32_t> parent;  // aggregate of each row
     int64_t n_coarse = 0;
-    std::unique_ptr<Mat> P;     // null where the caller will not use it (too little coarsening)
+    std::unique_ptr<Mat> P;       // null where the caller will not use it (too little coarsening)
 };
 
 // automatic depth: a level that shrinks by less than 4:3 is a stall
@@ -409,14 +409,18 @@ bool agglomerate_device(const Mat &A, int64_t bmax, double weight, bool additive
     out.n_coarse = centres + (both >> 32);
     if (out.n_coarse < 1 || (drop_stalled && stalls(n, out.n_coarse))) return true;
     out.P = make_csr_device(ctx, n, out.n_coarse, nnz, UGPU_F64);
-    out.parent.alloc(sizeof(int32_t) * n);
+    Buffer parent;
+    parent.alloc(sizeof(int32_t) * n);
     k_agg_prolongator<<<stream_grid(ctx, n), kBlock, 0, ctx.stream>>>(
         word.as<unsigned long long>(), id.as<int64_t>(), h.excluded ? kept.as<int64_t>() : nullptr, nnz, centres, n,
-        a_max.as<double>(), out.parent.as<int32_t>(), out.P->rowptr.as<int32_t>(), out.P->colidx.as<int32_t>(),
+        a_max.as<double>(), parent.as<int32_t>(), out.P->rowptr.as<int32_t>(), out.P->colidx.as<int32_t>(),
         out.P->vals.as<double>());
     ctx.launches++;
     UGPU_LAUNCH_CHECK();
+    out.parent.resize(size_t(n));
+    UGPU_CUDA(cudaMemcpyAsync(out.parent.data(), parent.ptr, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, ctx.stream));
     finalize_matrix(*out.P);
+    UGPU_CUDA(cudaStreamSynchronize(ctx.stream));
     return true;
 }
 
@@ -518,10 +522,8 @@ public:
             // dominate the cycle)
             if (want_levels == 0 && stalls(cur->nrows, g.n_coarse)) break;
             if (!g.P) {
-                g.parent.alloc(sizeof(int32_t) * cur->nrows);
-                UGPU_CUDA(cudaMemcpyAsync(g.parent.ptr, parent.data(), sizeof(int32_t) * cur->nrows,
-                                          cudaMemcpyHostToDevice, ctx->stream));
-                g.P = prolongator(*ctx, cur->nrows, g.n_coarse, parent, amax);  // waits for the stream
+                g.P = prolongator(*ctx, cur->nrows, g.n_coarse, parent, amax);
+                g.parent = parent;
             }
             auto P = std::move(g.P);
             parents_.push_back(std::move(g.parent));
@@ -549,14 +551,13 @@ public:
 
     int n_transfers() const { return int(transfers_.size()); }
     int64_t coarse_rows(int l) const { return transfers_.at(size_t(l))->ncols; }
-    int64_t fine_rows(int l) const { return transfers_.at(size_t(l))->nrows; }
-    const Buffer &parent(int l) const { return parents_.at(size_t(l)); }
+    const std::vector<int32_t> &parent(int l) const { return parents_.at(size_t(l)); }
     const Solver *multigrid() const { return mg_.get(); }
 
 private:
     std::unique_ptr<Solver> mg_;
     std::vector<std::unique_ptr<Mat>> transfers_;  // fine -> coarse, as built
-    std::vector<Buffer> parents_;
+    std::vector<std::vector<int32_t>> parents_;
 };
 
 std::unique_ptr<Solver> make_amg(Context *c) { return std::make_unique<AlgebraicMultigrid>(c); }
@@ -576,13 +577,10 @@ int ugpu_amg_parent(const ugpu_solver *amg, int level, int32_t *parent, int64_t 
     auto *a = dynamic_cast<const ugpu::AlgebraicMultigrid *>(amg->impl.get());
     UGPU_CHECK(a, UGPU_ERR_ARG, "not an algebraic multigrid solver");
     UGPU_CHECK(level >= 0 && level < a->n_transfers(), UGPU_ERR_ARG, "level out of range");
-    if (n) *n = a->fine_rows(level);
+    const auto &p = a->parent(level);
+    if (n) *n = int64_t(p.size());
     if (n_coarse) *n_coarse = a->coarse_rows(level);
-    if (parent) {
-        UGPU_CUDA(cudaMemcpyAsync(parent, a->parent(level).ptr, sizeof(int32_t) * a->fine_rows(level),
-                                  cudaMemcpyDeviceToHost, a->ctx->stream));
-        UGPU_CUDA(cudaStreamSynchronize(a->ctx->stream));
-    }
+    if (parent) std::copy(p.begin(), p.end(), parent);
     UGPU_ABI_END(amg->impl->ctx)
 }
 
