@@ -460,8 +460,14 @@ __global__ void __launch_bounds__(256) k_gemv64_split(const double *M, int64_t n
     extern __shared__ __align__(16) double sr[];  // r in FP64
     __shared__ double part[8];
     if (done && *done) return;
-#pragma unroll 8
-    for (int64_t j = threadIdx.x; j < n; j += 256) sr[j] = cvt<double>(__ldg(r + j));
+    for (int64_t j0 = threadIdx.x; j0 < n; j0 += 8 * 256) {
+        VT v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = j0 + u * 256 < n ? __ldg(r + j0 + u * 256) : VT(0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (j0 + u * 256 < n) sr[j0 + u * 256] = cvt<double>(v[u]);
+    }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rl = warp >> 1, q = warp & 1;  // row of the four, half of the row
@@ -474,16 +480,28 @@ __global__ void __launch_bounds__(256) k_gemv64_split(const double *M, int64_t n
                 const int64_t n2 = n >> 1, c0 = q * n2 / 2, c1 = (q + 1) * n2 / 2;
                 const double2 *rv = reinterpret_cast<const double2 *>(row);
                 const double2 *xv = reinterpret_cast<const double2 *>(sr);
-#pragma unroll 8
-                for (int64_t c = c0 + lane; c < c1; c += 32) {
-                    const double2 a = __ldg(rv + c), b = xv[c];
-                    s0 = fma(a.x, b.x, s0);
-                    s1 = fma(a.y, b.y, s1);
+                for (int64_t k = c0 + lane; k < c1; k += 8 * 32) {
+                    double2 a[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) a[u] = k + u * 32 < c1 ? __ldg(rv + k + u * 32) : make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (k + u * 32 >= c1) break;
+                        const double2 b = xv[k + u * 32];
+                        s0 = fma(a[u].x, b.x, s0);
+                        s1 = fma(a[u].y, b.y, s1);
+                    }
                 }
             } else {
                 const int64_t c0 = q * n / 2, c1 = (q + 1) * n / 2;
-#pragma unroll 8
-                for (int64_t c = c0 + lane; c < c1; c += 32) s0 = fma(__ldg(row + c), sr[c], s0);
+                for (int64_t k = c0 + lane; k < c1; k += 8 * 32) {
+                    double a[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) a[u] = k + u * 32 < c1 ? __ldg(row + k + u * 32) : 0.0;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (k + u * 32 < c1) s0 = fma(a[u], sr[k + u * 32], s0);
+                }
             }
         }
         const double s = warp_sum(s0 + s1);
