@@ -296,6 +296,93 @@ def test_cholesky_products_around_the_fp64_tiles(ctx, n):
     assert rel(x.numpy(), y) <= 1.2e-12
 
 
+def _contrast_box(dims, kind, offsets=((1, 0, 0), (0, 1, 0), (0, 0, 1))):
+    """-div(k grad u) on a box by differences along `offsets`, k per cell with little or strong contrast."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(5)
+    n = int(np.prod(dims))
+    k = {"poisson": np.ones(n), "lognormal": rng.lognormal(0, 1, n), "strong": rng.lognormal(0, 4, n),
+         "jumps": np.where(rng.random(n) < 0.5, 1.0, 1e8)}[kind]
+    i = np.arange(n)
+    at = [i % dims[0], i // dims[0] % dims[1], i // (dims[0] * dims[1])]
+    r, c, v, diag = [], [], [], k.copy()
+    for o in offsets:
+        ok = np.all([(p + q >= 0) & (p + q < d) for p, q, d in zip(at, o, dims)], axis=0)
+        a = i[ok]
+        b = a + o[0] + dims[0] * (o[1] + dims[1] * o[2])
+        w = 2 * k[a] * k[b] / (k[a] + k[b])
+        r, c, v = r + [a, b], c + [b, a], v + [-w, -w]
+        np.add.at(diag, a, w)
+        np.add.at(diag, b, w)
+    A = sp.csr_matrix((np.concatenate(v + [diag]), (np.concatenate(r + [i]), np.concatenate(c + [i]))), shape=(n, n))
+    A.sort_indices()
+    return A
+
+
+def _extended_columns(A, cols):
+    """Columns of A^-1 by banded elimination in extended precision."""
+    n = A.shape[0]
+    M = A.tocoo()
+    w = int(np.abs(M.row - M.col).max())
+    D = np.zeros((n + w, n + w) if n < 200 else (n, n), dtype=np.longdouble)[:n, :n]
+    D[M.row, M.col] = M.data
+    X = np.zeros((n, len(cols)), dtype=np.longdouble)
+    X[cols, np.arange(len(cols))] = 1
+    for k in range(n):
+        e = min(n, k + w + 1)
+        f = D[k + 1:e, k] / D[k, k]
+        D[k + 1:e, k:e] -= f[:, None] * D[k, k:e]
+        X[k + 1:e] -= f[:, None] * X[k]
+    for k in range(n - 1, -1, -1):
+        e = min(n, k + w + 1)
+        X[k] = (X[k] - D[k, k + 1:e] @ X[k + 1:e]) / D[k, k]
+    return X
+
+
+@pytest.mark.parametrize("kind", ["poisson", "lognormal", "strong", "jumps"])
+@pytest.mark.parametrize("dims", [(8, 8, 8), (27, 19, 1), (10, 10, 10), (11, 13, 9), (12, 12, 12)])
+def test_cholesky_entries_keep_their_relative_accuracy(ctx, dims, kind):
+    """Point sources: every entry of the solution, however far below the largest, is right to n eps, the bound of an
+    FP64 elimination of an M-matrix (no cancellation), on both sides of the row count where the products move
+    to the tensor cores."""
+    A = _contrast_box(dims, kind)
+    n = A.shape[0]
+    cols = [0, n // 2]
+    ref = _extended_columns(A, cols)
+    s = U.CholeskySolver(ctx)
+    s.update(U.SparseMatrix(ctx, P.CSR.from_scipy(A)))
+    for q, c in enumerate(cols):
+        b = np.zeros(n)
+        b[c] = 1.0
+        x = U.Vector(ctx, n=n)
+        s.apply(U.Vector(ctx, b), x)
+        assert np.abs((x.numpy() - ref[:, q]) / ref[:, q]).max() <= n * 2.0 ** -52
+
+
+def test_cholesky_forms_of_the_operator(ctx):
+    """What the factorisation reads is the lower triangle: an operator without its upper one, one whose upper
+    one differs, and a wide row; an indefinite operator is refused at sizes of both kinds of products."""
+    import scipy.sparse as sp
+
+    A = _contrast_box((10, 10, 10), "lognormal", ((1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 1), (1, -1, 0)))
+    n = A.shape[0]
+    y = np.random.default_rng(1).standard_normal(n)
+    up = sp.triu(A, 1).tocsr()
+    arrow = sp.csr_matrix((np.full(n, 1e-3), (np.zeros(n, dtype=int), np.arange(n))), shape=(n, n))
+    full = (A + arrow + arrow.T).tocsr()  # smallest eigenvalue of A 0.73, norm of the arrow 0.032
+    for M, S in ((sp.tril(A).tocsr(), A), ((A + 0.25 * up).tocsr(), A), (full, full)):
+        M.sort_indices()
+        x = U.Vector(ctx, n=n)
+        U.CholeskySolver(ctx).solve(U.SparseMatrix(ctx, P.CSR.from_scipy(M)), U.Vector(ctx, S @ y), x)
+        assert rel(x.numpy(), y) <= 1e-10  # cond 100, times n eps, and some
+    for m in (400, n):
+        B = A[:m, :m].tolil()
+        B[m - 2, m - 2] = -1.0
+        with pytest.raises(U.UgpuError, match="positive definite"):
+            U.CholeskySolver(ctx).update(U.SparseMatrix(ctx, P.CSR.from_scipy(B.tocsr())))
+
+
 def test_cholesky_solver_factored_inverse_above_4096(ctx):
     """Coarse sizes above 4096 keep the inverse factored (Y = L^-1 and Y^T in one buffer, two
     triangular GEMVs per solve): FP64 and FP32 vectors against a direct solve."""

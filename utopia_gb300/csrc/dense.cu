@@ -9,10 +9,11 @@
 // A^-1 = Y^T Y is formed.  Every coarse solve is then one
 // FP64 GEMV with A^-1, an L2-resident matrix for the coarse sizes of the hot path
 // (1728^2 and 4096^2 doubles), instead of two latency-bound triangular sweeps.
-// GB300's FP64 tensor rate is no higher than its FP64 FMA rate, so the set-up's products run on
-// the FP16 tensor cores by exact splitting (gemm64.cu); only the 64 x 64 diagonal blocks use the
-// FP64 pipe.
+// GB300's FP64 tensor rate is no higher than its FP64 FMA rate, so the set-up's large products run on
+// the FP16 tensor cores by splitting (gemm64.cu) and the inverse is refined to FP64's accuracy entry by entry; the
+// small products, the 64 x 64 diagonal blocks, and the set-ups that cannot be refined use the FP64 pipe.
 #include <cmath>
+#include <cstring>
 #include <functional>
 
 #include "abi_util.cuh"
@@ -210,9 +211,10 @@ __global__ void __launch_bounds__(256) k_chol_inv_block(const double *A, double 
 
 // The result from its lower triangle, with the scaling of the operator undone: the inverse
 // (D A D)^-1 -> A^-1 = D (D A D)^-1 D with its upper triangle mirrored (rows scaled too), or L^-1 -> L^-1 D with its
-// transpose in the upper triangle.  32 x 32 tiles through shared memory, so that both triangles are
-// written in whole lines.
-__global__ void __launch_bounds__(256) k_unscale_mirror(double *A, int64_t n, const int *h, int rows_too) {
+// transpose in the upper triangle.  h null: mirrored as it is.  add (may be null) is added to the lower triangle
+// first.  32 x 32 tiles through shared memory, so that both triangles are written in whole lines.
+__global__ void __launch_bounds__(256) k_unscale_mirror(double *A, const double *add, int64_t n, const int *h,
+                                                        int rows_too) {
     if (blockIdx.x > blockIdx.y) return;
     __shared__ double s[32][33];
     const int64_t i0 = 32 * int64_t(blockIdx.y), j0 = 32 * int64_t(blockIdx.x);
@@ -221,7 +223,9 @@ __global__ void __launch_bounds__(256) k_unscale_mirror(double *A, int64_t n, co
         const int64_t i = i0 + r, j = j0 + tx;
         double v = 0.0;
         if (i < n && j <= i) {
-            v = scale_pow2(A[i * n + j], -h[j] - (rows_too ? h[i] : 0));
+            v = A[i * n + j];
+            if (add) v += add[i * n + j];
+            if (h) v = scale_pow2(v, -h[j] - (rows_too ? h[i] : 0));
             A[i * n + j] = v;
         }
         s[r][tx] = v;
@@ -231,6 +235,85 @@ __global__ void __launch_bounds__(256) k_unscale_mirror(double *A, int64_t n, co
         const int64_t i = j0 + r, j = i0 + tx;  // the mirrored entry (i, j), j > i
         if (j < n && j > i) A[i * n + j] = s[tx][r];
     }
+}
+
+// The entries of D A D with both triangles taken from the lower one, as the factorisation takes them; a warp per row.
+// *one_sided: some entry of the lower triangle has no place in the upper one.
+template <class V>
+__global__ void __launch_bounds__(kBlock) k_symmetric_values(const int32_t *rp, const int32_t *ci, const V *cv, int64_t n,
+                                                             const int *h, double *sv, int *one_sided) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = int64_t(gridDim.x) * blockDim.x / 32;
+    for (int64_t i = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / 32; i < n; i += nw)
+        for (int32_t k = rp[i] + lane; k < rp[i + 1]; k += 32) {
+            const int32_t c = ci[k];
+            int32_t e = k;
+            if (c != i) {
+                const int32_t e1 = rp[c + 1];
+                for (e = rp[c]; e < e1 && ci[e] != i; ++e) {
+                }
+                if (e == e1) e = -1;
+            }
+            if (c < i && e < 0) atomicOr(one_sided, 1);
+            const int32_t from = c <= i ? k : e;
+            sv[k] = from < 0 ? 0.0 : scale_pow2(cvt<double>(cv[from]), -h[i] - h[c]);
+        }
+}
+
+// |v| as binary32 by truncation; 0 below its normal numbers, infinity above them and for NaN
+__device__ __forceinline__ float abs32(double v) {
+    const uint32_t h = uint32_t(__double2hiint(v)) & 0x7fffffffu;
+    if (h < (897u << 20)) return 0.0f;
+    if (h >= (1150u << 20)) return __int_as_float(0x7f800000);
+    return __uint_as_float(__funnelshift_l(uint32_t(__double2loint(v)), h - (896u << 20), 3));
+}
+
+// R = I - S X and *worst = max |R_kj| / (|S| |X|)_kj (bits of a binary32; infinity where that is no number).  A CTA takes
+// 512 columns of one row, lanes along the row.  EXACT: the sums in twice FP64's precision (Ogita, Rump and Oishi,
+// "Accurate sum and dot product", 2005: error-free products and additions), ten FP64 operations for one.
+template <bool EXACT>
+__global__ void __launch_bounds__(256) k_inverse_residual(const int32_t *rp, const int32_t *ci, const double *sv, int64_t n,
+                                                          const double *X, double *R, unsigned int *worst) {
+    const int64_t i = blockIdx.y;
+    const int64_t j0 = int64_t(blockIdx.x) * 512 + threadIdx.x;
+    const int32_t e0 = rp[i], e1 = rp[i + 1];
+    float bad = 0.0f;
+    double r[2], low[2] = {0.0, 0.0};
+    float size[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) r[q] = j0 + 256 * q == i ? 1.0 : 0.0;
+#pragma unroll 4
+    for (int32_t e = e0; e < e1; ++e) {
+        const double a = __ldg(sv + e);
+        const double *x = X + int64_t(__ldg(ci + e)) * n;
+        const float a32 = abs32(a);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double v = j0 + 256 * q < n ? __ldg(x + j0 + 256 * q) : 0.0;
+            if constexpr (EXACT) {
+                const double p = -a * v, pe = fma(-a, v, -p);
+                const double s = r[q] + p, b = s - r[q];
+                low[q] += ((r[q] - (s - b)) + (p - b)) + pe;
+                r[q] = s;
+            } else {
+                r[q] = fma(-a, v, r[q]);
+            }
+            size[q] = fmaf(a32, abs32(v), size[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        if (j0 + 256 * q >= n) continue;
+        const double v = EXACT ? r[q] + low[q] : r[q];
+        R[i * n + j0 + 256 * q] = v;
+        const float v32 = abs32(v);
+        if (v32 > 0.0f) {
+            const float w = __fdividef(v32, size[q]);
+            bad = fmaxf(bad, w >= 0.0f && size[q] < 1e37f && v32 < 1e37f ? w : __int_as_float(0x7f800000));
+        }
+    }
+    const unsigned int m = __reduce_max_sync(0xffffffffu, __float_as_uint(bad));
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(worst, m);
 }
 
 __global__ void k_zero(double *p, int64_t m) {
@@ -286,42 +369,73 @@ void DenseCholesky::make_fp32_inverse() {
     if (n) launch_convert(*ctx, Ainv.ptr, UGPU_F64, Ainv32.ptr, UGPU_F32, n * n);
 }
 
+// Row count above which the products run on the tensor cores (7 points: 512 rows 0.88 ms against 0.92 with FP64
+// multiply-adds, 729 rows 1.43 / 1.76, 1728 rows 3.8 / 11.4, 4096 rows 14.0 / 74.6; 343 rows 0.64 / 0.62).
+constexpr int64_t kSplitMin = 512;
+// max |R| / (|S| |X|) of an inverse X (R = I - S X) up to which one correction by an FP64 residual ends the refinement
+// (what the split products leave on operators of little contrast); up to which X needs none, in units of
+// sqrt(n) eps (FP64 multiply-adds left 0.48 to 17 of them on 60 coarse operators of 528 to 4096 rows, the median
+// 0.7); and up to which a correction by an exact residual is the last one.
+constexpr double kMild = 0x1p-33, kSettled = 0.5, kLast = 0x1p-40;
+constexpr int kExactSteps = 4;
+
 bool DenseCholesky::factor(const Mat &A) {
     UGPU_CHECK(A.nrows == A.ncols, UGPU_ERR_ARG, "coarse solver: square matrix required");
-    Context &c = *A.ctx;
-    ctx = &c;
+    ctx = A.ctx;
     n = A.nrows;
     UGPU_CHECK(n <= 16384, UGPU_ERR_UNSUPPORTED, "coarse solver: dense size limited to 16384");
+    tri = n > kDenseTriMin;
+    // Split products on the tensor cores where the inverse can be refined: formed explicitly, by a sparse operator
+    // (the residual's n nnz FMAs stay below a quarter of the inverse's).  What they call indefinite or what
+    // does not settle is decided by FP64 multiply-adds.
+    if (n > kSplitMin && !tri && A.nnz <= n * n / 8 && invert(A, false)) return true;
+    return invert(A, true);
+}
+
+// fma: FP64 multiply-adds throughout.  Otherwise the large products are split ones, each accurate to rounding in its
+// rows' maxima only: small entries of the inverse (a decaying row, a jump in the coefficients) are lost below them.
+// So X is refined, X + X (I - S X): the residual carries every entry's relative error, whatever its size, and the
+// correction is small beside X.  One correction, which the residual of the result has to confirm unless the
+// operator is mild; where it does not, corrections by exact residuals.  Worst relative error of an entry, operators
+// of 1000 rows, FP64 multiply-adds / split / refined: Poisson 4e-15 / 7e-13 / 1e-15, lognormal sigma 1
+// 4e-15 / 1e-11 / 1e-15, sigma 4 1e-14 / 2e-6 / 2e-16, coefficients 1 and 1e8 5e-15 / 1 / 3e-16.
+bool DenseCholesky::invert(const Mat &A, bool fma) {
+    Context &c = *A.ctx;
     L.alloc(sizeof(double) * std::max<int64_t>(n * n, 1));
     Ainv.alloc(sizeof(double) * std::max<int64_t>(n * n, 1));
     Ainv32.release();
     if (n == 0) return true;
     double *Lp = L.as<double>();
     double *Y = Ainv.as<double>();  // holds L^-1 first
+    const int32_t *rp = A.rowptr.as<int32_t>(), *ci = A.colidx.as<int32_t>();
     Buffer hx;  // half exponents of the diagonal
     hx.alloc(sizeof(int) * size_t(n));
     const dim3 tiles(unsigned((n + 31) / 32), unsigned((n + 31) / 32));
+    Buffer state;  // [0] not definite, [1] an entry without its mirror image, [2] the residual's measure
+    state.alloc(3 * sizeof(int));
+    UGPU_CUDA(cudaMemsetAsync(state.ptr, 0, 3 * sizeof(int), c.stream));
+    int *bad = state.as<int>();
+    Buffer sv;  // the entries of D A D
+    if (!fma) sv.alloc(sizeof(double) * size_t(std::max<int64_t>(A.nnz, 1)));
     auto dens = [&](auto tag) {
         using V = decltype(tag);
-        k_half_exponents<V><<<stream_grid(c, n), kBlock, 0, c.stream>>>(A.rowptr.as<int32_t>(), A.colidx.as<int32_t>(),
-                                                                        A.vals.as<V>(), n, hx.as<int>());
-        k_densify<V><<<int(std::min<int64_t>(n, 4096)), 256, 0, c.stream>>>(A.rowptr.as<int32_t>(),
-                                                                              A.colidx.as<int32_t>(), A.vals.as<V>(),
-                                                                              n, hx.as<int>(), Lp);
+        k_half_exponents<V><<<stream_grid(c, n), kBlock, 0, c.stream>>>(rp, ci, A.vals.as<V>(), n, hx.as<int>());
+        k_densify<V><<<int(std::min<int64_t>(n, 4096)), 256, 0, c.stream>>>(rp, ci, A.vals.as<V>(), n, hx.as<int>(), Lp);
+        c.launches += 2;
+        if (fma) return;
+        k_symmetric_values<V><<<stream_grid(c, 32 * n), kBlock, 0, c.stream>>>(rp, ci, A.vals.as<V>(), n, hx.as<int>(),
+                                                                              sv.as<double>(), bad + 1);
+        c.launches++;
     };
     if (A.vdtype == UGPU_F64) dens(double{});
     else if (A.vdtype == UGPU_F32) dens(float{});
     else dens(__nv_bfloat16{});
-    c.launches += 2;
     UGPU_LAUNCH_CHECK();
-    Buffer bad;
-    bad.alloc(sizeof(int));
-    UGPU_CUDA(cudaMemsetAsync(bad.ptr, 0, sizeof(int), c.stream));
     // Factorisation and inversion by recursive halving at multiples of NB: with A11 = L11 L11^T and
     // Y11 = L11^-1 known, L21 = A21 Y11^T, A22 -= L21 L21^T, then the same for A22, and
     // Y21 = -Y22 (L21 Y11).  Every product is a GEMM of the current half's size (gemm64.cu), the
     // triangular factors' zero parts left out; L21 Y11 takes A21's place (L itself is not needed once Y is).
-    // Measured with the inverse: 4096 rows 10.6 ms, 1728 rows 3.3 ms (FP64 tiles: 141 and 22.5 ms).
+    // With the inverse, before its refinement: 4096 rows 10.6 ms, 1728 rows 3.3 ms.
     k_zero<<<stream_grid(c, n * n), kBlock, 0, c.stream>>>(Y, n * n);
     c.launches++;
     Buffer T, scales;
@@ -330,7 +444,7 @@ bool DenseCholesky::factor(const Mat &A) {
     double *Tp = T.as<double>();
     std::function<void(int64_t, int64_t)> chol_inv = [&](int64_t r0, int64_t m) {
         if (m <= NB) {
-            k_chol_inv_block<<<1, 256, 0, c.stream>>>(Lp, Y, n, r0, int(m), bad.as<int>());
+            k_chol_inv_block<<<1, 256, 0, c.stream>>>(Lp, Y, n, r0, int(m), bad);
             c.launches++;
             return;
         }
@@ -339,6 +453,7 @@ bool DenseCholesky::factor(const Mat &A) {
         const double *Y11 = Y + r0 * n + r0, *Y22 = Y + (r0 + h) * n + r0 + h;
         chol_inv(r0, h);
         Gemm64 g;
+        g.fma = fma;
         g.M = int(m2), g.N = int(h), g.K = int(h);  // T = L21 = A21 Y11^T
         g.A = A21, g.a_row = n, g.a_k = 1;
         g.B = Y11, g.b_row = n, g.b_k = 1;
@@ -369,35 +484,76 @@ bool DenseCholesky::factor(const Mat &A) {
     };
     chol_inv(0, n);
     UGPU_LAUNCH_CHECK();
-    int hbad = 0;
-    UGPU_CUDA(cudaMemcpyAsync(&hbad, bad.ptr, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.check_kernel_flags();
-    if (hbad) return false;
-    tmp_d.ensure(sizeof(double) * size_t(n));
-    tri = n > kDenseTriMin;
-    if (tri) {  // Y in the lower triangle, Y^T in the upper one
-        k_unscale_mirror<<<tiles, 256, 0, c.stream>>>(Y, n, hx.as<int>(), 0);
+    int hs[3] = {0, 0, 0};
+    auto read_state = [&] {
+        UGPU_CUDA(cudaMemcpyAsync(hs, state.ptr, sizeof(hs), cudaMemcpyDeviceToHost, c.stream));
+        c.check_kernel_flags();
+    };
+    auto mirror = [&](double *M, const double *add, const int *h, int rows_too) {
+        k_unscale_mirror<<<tiles, 256, 0, c.stream>>>(M, add, n, h, rows_too);
         c.launches++;
         UGPU_LAUNCH_CHECK();
+    };
+    tmp_d.ensure(sizeof(double) * size_t(n));
+    if (tri) {  // Y in the lower triangle, Y^T in the upper one
+        read_state();
+        if (hs[0]) return false;
+        mirror(Y, nullptr, hx.as<int>(), 0);
         UGPU_CUDA(cudaStreamSynchronize(c.stream));
         return true;
     }
-    // Ainv = Y^T Y (stored in L's buffer, then swapped): the lower triangle's tiles, then mirrored
+    // A^-1 = Y^T Y (stored in L's buffer, then swapped): the lower triangle's tiles, then mirrored
     // (the product is symmetric bit for bit: (i, j) and (j, i) sum the same products in one order)
-    {
-        Gemm64 g;
-        g.M = g.N = g.K = int(n);
-        g.A = Y, g.a_row = 1, g.a_k = n;
-        g.B = Y, g.b_row = 1, g.b_k = n;
-        g.C = Lp, g.ldc = n;
-        g.flags = kGemmLower | kGemmKFromM | kGemmKFromN;
-        gemm64(c, g, scales);
-        k_unscale_mirror<<<tiles, 256, 0, c.stream>>>(Lp, n, hx.as<int>(), 1);
-        c.launches++;
-        UGPU_LAUNCH_CHECK();
+    Gemm64 g;
+    g.fma = fma;
+    g.M = g.N = g.K = int(n);
+    g.A = Y, g.a_row = 1, g.a_k = n;
+    g.B = Y, g.b_row = 1, g.b_k = n;
+    g.C = Lp, g.ldc = n;
+    g.flags = kGemmLower | kGemmKFromM | kGemmKFromN;
+    gemm64(c, g, scales);
+    if (fma) {
+        mirror(Lp, nullptr, hx.as<int>(), 1);
+        read_state();
+        if (hs[0]) return false;
+    } else {
+        Buffer correction;
+        correction.alloc(sizeof(double) * size_t(n * n));
+        mirror(Lp, nullptr, nullptr, 0);
+        g.A = Lp, g.a_row = n, g.a_k = 1;  // X R, R in Y's place
+        g.C = correction.as<double>();
+        g.flags = kGemmLower;
+        const dim3 rows(unsigned((n + 511) / 512), unsigned(n));
+        auto residual = [&](bool exact) {
+            UGPU_CUDA(cudaMemsetAsync(bad + 2, 0, sizeof(int), c.stream));
+            auto *kernel = exact ? k_inverse_residual<true> : k_inverse_residual<false>;
+            kernel<<<rows, 256, 0, c.stream>>>(rp, ci, sv.as<double>(), n, Lp, Y, reinterpret_cast<unsigned int *>(bad + 2));
+            c.launches++;
+            UGPU_LAUNCH_CHECK();
+            read_state();
+            float worst;
+            memcpy(&worst, &hs[2], sizeof(worst));
+            return double(worst);
+        };
+        auto correct = [&] {
+            gemm64(c, g, scales);
+            mirror(Lp, correction.as<double>(), nullptr, 0);
+        };
+        double worst = residual(false);
+        if (hs[0] || hs[1] || !(worst < HUGE_VAL)) return false;
+        correct();
+        if (worst > kMild && !(residual(false) <= kSettled * std::sqrt(double(n)) * 0x1p-52))
+            for (int k = 0;; ++k) {
+                const double before = worst;
+                worst = residual(true);
+                if (!(worst < 0.25 * before) || k == kExactSteps) return false;
+                correct();
+                if (worst <= kLast) break;
+            }
+        mirror(Lp, nullptr, hx.as<int>(), 1);
+        c.check_kernel_flags();
     }
-    std::swap(L, Ainv);  // Ainv now holds the inverse; L holds L^-1 (kept for diagnostics)
-    c.check_kernel_flags();
+    std::swap(L, Ainv);  // Ainv now holds the inverse
     return true;
 }
 

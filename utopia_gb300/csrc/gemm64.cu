@@ -18,8 +18,11 @@
 // the next 32 values into the other stage; every fourth stage all threads read the accumulators into
 // their integers.  Bound by the issue slots of the splitting (about 10 k instructions of 16 warps per stage)
 // beside the MMAs (tensor pipe 35 % busy).  Measured: 4096^3 in 5.7 ms (24 TFLOP/s of FP64 results) where FP64
-// FMA tiles took about 130 ms (1.05 TFLOP/s), 1024^3 in 0.12 ms; the error against 113-bit sums is at or below
-// that of an FMA chain (1.9e-16 against 1.2e-15 of max max sqrt(K) at K = 300).
+// FMA tiles took about 130 ms (1.05 TFLOP/s), 1024^3 in 0.12 ms.
+// The error is absolute in the two rows' maxima: K 2^-57 max|a| max|b| bounds it (random operands, K = 300:
+// 1.9e-16 of max max sqrt(K), an FMA chain 1.2e-15).  A sum of much smaller products, a row's small entries against
+// small ones, has no relative accuracy below that, where an FMA chain's holds for any scale: who takes a
+// split product has to restore it (dense.cu refines the inverse) or ask for FP64 multiply-adds (Gemm64::fma).
 #include "abi_util.cuh"
 #include "device_util.cuh"
 #include "gemm64.cuh"
@@ -470,6 +473,67 @@ __global__ void __launch_bounds__(256) k_gemm64_small(const Gemm64 g) {
     *C = g.add ? *C + acc : acc;
 }
 
+// Larger products where every product has to be an FP64 multiply-add: T x T tiles, 16 x 16 threads of T / 16 x T / 16
+// outputs.  Bound by the FP64 pipes (1.05 TFLOP/s at 4096^3).
+template <bool AK, bool BK, int T>
+__global__ void __launch_bounds__(256) k_gemm64_fma(const Gemm64 g) {
+    constexpr int TK = 16, PT = T / 16;
+    __shared__ double s_a[TK][T + 1], s_b[TK][T + 1];
+    const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
+    if ((g.flags & kGemmLower) && n0 > m0 + T - 1) return;
+    int k0 = 0, k1 = g.K;
+    if (g.flags & kGemmKFromN) k0 = max(k0, n0);
+    if (g.flags & kGemmKFromM) k0 = max(k0, m0);
+    if (g.flags & kGemmKToN) k1 = min(k1, n0 + T);
+    if (g.flags & kGemmKToM) k1 = min(k1, m0 + T);
+    const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+    double acc[PT][PT] = {};
+    for (int k = k0; k < k1; k += TK) {
+        for (int e = t; e < T * TK; e += 256) {
+            const int ra = AK ? e / TK : e % T, ka = AK ? e % TK : e / T;
+            const int rb = BK ? e / TK : e % T, kb = BK ? e % TK : e / T;
+            s_a[ka][ra] = m0 + ra < g.M && k + ka < k1 ? __ldg(g.A + (m0 + ra) * g.a_row + (k + ka) * g.a_k) : 0.0;
+            s_b[kb][rb] = n0 + rb < g.N && k + kb < k1 ? __ldg(g.B + (n0 + rb) * g.b_row + (k + kb) * g.b_k) : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < TK; ++q) {
+            double a[PT], b[PT];
+#pragma unroll
+            for (int i = 0; i < PT; ++i) {
+                a[i] = s_a[q][ty + 16 * i];
+                b[i] = s_b[q][tx + 16 * i];
+            }
+#pragma unroll
+            for (int i = 0; i < PT; ++i)
+#pragma unroll
+                for (int j = 0; j < PT; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < PT; ++i)
+#pragma unroll
+        for (int j = 0; j < PT; ++j) {
+            const int r = m0 + ty + 16 * i, c = n0 + tx + 16 * j;
+            if (r >= g.M || c >= g.N) continue;
+            double *o = g.C + int64_t(r) * g.ldc + c;
+            const double v = g.negate ? -acc[i][j] : acc[i][j];
+            *o = g.add ? *o + v : v;
+        }
+}
+
+// the tile that keeps the grid at least two CTAs per SM
+template <int T>
+void launch_fma(Context &c, const Gemm64 &g) {
+    const dim3 grid(unsigned((g.N + T - 1) / T), unsigned((g.M + T - 1) / T));
+    auto run = [&](auto kern) { kern<<<grid, 256, 0, c.stream>>>(g); };
+    if (g.a_k == 1 && g.b_k == 1) run(k_gemm64_fma<true, true, T>);
+    else if (g.a_k == 1) run(k_gemm64_fma<true, false, T>);
+    else if (g.b_k == 1) run(k_gemm64_fma<false, true, T>);
+    else run(k_gemm64_fma<false, false, T>);
+}
+
 }  // namespace
 
 void gemm64(Context &c, const Gemm64 &args, Buffer &scales) {
@@ -485,6 +549,13 @@ void gemm64(Context &c, const Gemm64 &args, Buffer &scales) {
     if (g.K <= kSmallK && int64_t(g.M) * g.N * g.K <= kSmallWork) {
         const dim3 tiles(unsigned((g.N + kSmallTile - 1) / kSmallTile), unsigned((g.M + kSmallTile - 1) / kSmallTile));
         k_gemm64_small<<<tiles, 256, 0, c.stream>>>(g);
+        c.launches++;
+        UGPU_LAUNCH_CHECK();
+        return;
+    }
+    if (g.fma) {
+        if (int64_t((g.M + 63) / 64) * ((g.N + 63) / 64) >= 2 * int64_t(c.sms)) launch_fma<64>(c, g);
+        else launch_fma<32>(c, g);
         c.launches++;
         UGPU_LAUNCH_CHECK();
         return;

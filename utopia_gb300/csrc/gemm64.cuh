@@ -1,4 +1,4 @@
-// FP64 matrix products on the tensor cores (gemm64.cu).
+// FP64 matrix products, on the tensor cores or the FP64 pipes (gemm64.cu).
 #pragma once
 #include "internal.cuh"
 
@@ -25,6 +25,7 @@ struct Gemm64 {
     double *C = nullptr;
     int64_t ldc = 0;
     int flags = 0;
+    bool fma = false;  // FP64 multiply-adds throughout: no split product
     int vec_a = 0, vec_b = 0;  // set by gemm64()
 };
 // scales: scratch of at least M + N 32-bit words, grown where it is smaller (stream-ordered use)

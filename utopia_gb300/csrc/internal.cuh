@@ -393,6 +393,7 @@ struct DenseCholesky {
     Buffer Ainv32; // its FP32 copy for FP32 vectors (make_fp32_inverse; dropped by factor())
     Buffer tmp_d;  // FP64 rhs/solution staging
     bool factor(const Mat &A);           // returns false if not SPD
+    bool invert(const Mat &A, bool fma);  // one attempt of factor()
     void make_fp32_inverse();            // FP32 copy of the inverse (coarse solves with FP32 vectors)
     void solve(const void *rhs, int rdt, void *x, int xdt, const int *done = nullptr);
 };
