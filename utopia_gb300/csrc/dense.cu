@@ -372,11 +372,10 @@ void DenseCholesky::make_fp32_inverse() {
 // Row count above which the products run on the tensor cores (7 points: 512 rows 0.88 ms against 0.92 with FP64
 // multiply-adds, 729 rows 1.43 / 1.76, 1728 rows 3.8 / 11.4, 4096 rows 14.0 / 74.6; 343 rows 0.64 / 0.62).
 constexpr int64_t kSplitMin = 512;
-// max |R| / (|S| |X|) of an inverse X (R = I - S X) up to which one correction by an FP64 residual ends the refinement
-// (what the split products leave on operators of little contrast); up to which X needs none, in units of
-// sqrt(n) eps (FP64 multiply-adds left 0.48 to 17 of them on 60 coarse operators of 528 to 4096 rows, the median
-// 0.7); and up to which a correction by an exact residual is the last one.
-constexpr double kMild = 0x1p-33, kSettled = 0.5, kLast = 0x1p-40;
+// max |R| / (|S| |X|) of an inverse X (R = I - S X) up to which X needs no correction, in units of sqrt(n) eps (FP64
+// multiply-adds left 0.48 to 17 of them on 60 coarse operators of 528 to 4096 rows, the median 0.7), and up to
+// which a correction by an exact residual is the last one.
+constexpr double kSettled = 0.5, kLast = 0x1p-40;
 constexpr int kExactSteps = 4;
 
 bool DenseCholesky::factor(const Mat &A) {
@@ -395,8 +394,8 @@ bool DenseCholesky::factor(const Mat &A) {
 // fma: FP64 multiply-adds throughout.  Otherwise the large products are split ones, each accurate to rounding in its
 // rows' maxima only: small entries of the inverse (a decaying row, a jump in the coefficients) are lost below them.
 // So X is refined, X + X (I - S X): the residual carries every entry's relative error, whatever its size, and the
-// correction is small beside X.  One correction, which the residual of the result has to confirm unless the
-// operator is mild; where it does not, corrections by exact residuals.  Worst relative error of an entry, operators
+// correction is small beside X.  One correction, which the residual of the result has to confirm; where it does
+// not, corrections by exact residuals.  Worst relative error of an entry, operators
 // of 1000 rows, FP64 multiply-adds / split / refined: Poisson 4e-15 / 7e-13 / 1e-15, lognormal sigma 1
 // 4e-15 / 1e-11 / 1e-15, sigma 4 1e-14 / 2e-6 / 2e-16, coefficients 1 and 1e8 5e-15 / 1 / 3e-16.
 bool DenseCholesky::invert(const Mat &A, bool fma) {
@@ -542,7 +541,7 @@ bool DenseCholesky::invert(const Mat &A, bool fma) {
         double worst = residual(false);
         if (hs[0] || hs[1] || !(worst < HUGE_VAL)) return false;
         correct();
-        if (worst > kMild && !(residual(false) <= kSettled * std::sqrt(double(n)) * 0x1p-52))
+        if (!(residual(false) <= kSettled * std::sqrt(double(n)) * 0x1p-52))
             for (int k = 0;; ++k) {
                 const double before = worst;
                 worst = residual(true);
