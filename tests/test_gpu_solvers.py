@@ -296,6 +296,22 @@ def test_cholesky_products_around_the_fp64_tiles(ctx, n):
     assert rel(x.numpy(), y) <= 1.2e-12
 
 
+@pytest.mark.parametrize("n", [1, 63, 65, 256])
+@pytest.mark.parametrize("spread", [0, 400])
+def test_cholesky_pivots_are_rounded_once(ctx, n, spread):
+    """A diagonal operator's inverse is r r with r = 1 / sqrt(a): the root, the quotient and the square each rounded to
+    nearest, as on the host, with a brought into [1, 4) by an even power of two (which changes no rounding)."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(n + spread)
+    a = np.ldexp(rng.uniform(1.0, 4.0, n), 2 * rng.integers(-spread, spread + 1, n))
+    x = U.Vector(ctx, n=n)
+    U.CholeskySolver(ctx).solve(U.SparseMatrix(ctx, P.CSR.from_scipy(sp.diags(a).tocsr())), U.Vector(ctx, np.ones(n)), x)
+    h = (np.frexp(a)[1] - 1) >> 1
+    r = 1.0 / np.sqrt(np.ldexp(a, -2 * h))
+    np.testing.assert_array_equal(x.numpy(), np.ldexp(r * r, -2 * h))
+
+
 def _contrast_box(dims, kind, offsets=((1, 0, 0), (0, 1, 0), (0, 0, 1))):
     """-div(k grad u) on a box by differences along `offsets`, k per cell with little or strong contrast."""
     import scipy.sparse as sp

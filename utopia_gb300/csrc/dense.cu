@@ -63,27 +63,6 @@ __global__ void k_densify(const int32_t *rp, const int32_t *ci, const V *cv, int
     }
 }
 
-// 1 / v for v > 0 to FP64 rounding: the approximation instruction's estimate (about 20 bits) and one third-order
-// step of Householder's iteration, three FP64 instructions in a chain (the pivots of a block follow one another).
-__device__ __forceinline__ double rcp_pivot(double v) {
-    const int e = (__double2hiint(v) >> 20) - 1023;
-    if (e < -1000 || e > 1000) return 1.0 / v;  // subnormals, infinity, NaN, reciprocals near them
-    double r0;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(v));
-    const double d = fma(-v, r0, 1.0);
-    return fma(r0, fma(d, d, d), r0);
-}
-
-// 1 / sqrt(v) likewise, five FP64 instructions.
-__device__ __forceinline__ double rsqrt_pivot(double v) {
-    const int e = (__double2hiint(v) >> 20) - 1023;
-    if (e < -1000 || e > 1000) return 1.0 / sqrt(v);
-    double r0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(v));
-    const double d = fma(-(v * r0), r0, 1.0);
-    return fma(r0 * d, fma(d, 0.375, 0.5), r0);
-}
-
 // Cholesky of the kb x kb diagonal block at (k0, k0) of A (A = L L^T) and Y = L^-1, into Y's block.  Column c
 // of the remaining block and column c of the inverse share one array: entry (i, c) is A's remainder until
 // column c is eliminated, the inverse's entry after.  Eight columns at a time:
@@ -93,7 +72,7 @@ __device__ __forceinline__ double rsqrt_pivot(double v) {
 //   3. the rows below take the rank-8 update; warp 0 updates only the next pivot block and goes on to its
 //      elimination, a chain of dependent operations, while the other warps update the rest.
 // One CTA; bound by the FP64 pipe of one SM (87 k FMAs at two per clock, about 21 us) and what is left of the
-// chain: 56 us (62 with the other warps spread over all four schedulers).  Eliminating column by column with all
+// chain: 59 us (65 with the other warps spread over all four schedulers).  Eliminating column by column with all
 // warps queued the chain's operations behind the updates in that pipe (80-90 us); separate factorisation and
 // inversion kernels took 93 and 145 us.
 constexpr int PB = 8;
@@ -130,7 +109,7 @@ __global__ void __launch_bounds__(256) k_chol_inv_block(const double *A, double 
             // (l raw) beside the reciprocal: one operation follows it
             const double p0 = -l * (pc > j ? a0 : pc == j ? 1.0 : z0);
             const double p1 = -l * (pc + 1 > j ? a1 : pc + 1 == j ? 1.0 : z1);
-            const double inv = rcp_pivot(d);
+            const double inv = 1.0 / d;
             if (pr > j) {
                 m0 = fma(p0, inv, pc == j ? 0.0 : m0);
                 m1 = fma(p1, inv, pc + 1 == j ? 0.0 : m1);
@@ -140,7 +119,7 @@ __global__ void __launch_bounds__(256) k_chol_inv_block(const double *A, double 
                 if (pc + 1 == j) m1 = 1.0;
             }
         }
-        const double r = rsqrt_pivot(mine);
+        const double r = 1.0 / sqrt(mine);
         s_y[pr][pc] = pc <= pr ? m0 * r : 0.0;
         s_y[pr][pc + 1] = pc + 1 <= pr ? m1 * r : 0.0;
     };
