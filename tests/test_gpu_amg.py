@@ -40,6 +40,33 @@ def test_amg_hierarchy_matches_oracle(ctx, oracle, name):
         np.testing.assert_allclose(v, ov, rtol=1e-12, atol=1e-12 * np.abs(ov).max())
 
 
+@pytest.mark.parametrize("option", ["fix_semidefinite_operators", "keep_galerkin_structure"])
+@pytest.mark.parametrize("name", ["lognormal24", "random_graph"])
+def test_amg_galerkin_options(ctx, oracle, name, option):
+    """A small operator (diagonals below 1e-12 on some levels and rows): with fixed semidefinite levels every coarser
+    product is that of the fixed one, as in the oracle; a kept structure changes nothing."""
+    make, kw = CASES[name]
+    A = make()
+    i = np.repeat(np.arange(A.nrows), np.diff(A.rowptr))
+    scale = 1e-13 / np.median(A.values[i == A.colidx])
+    A = P.CSR(A.nrows, A.ncols, A.rowptr, A.colidx, A.values * scale)
+    kw = dict(kw, n_levels=4)
+    fix = option == "fix_semidefinite_operators"
+    Am = oracle.Matrix(A)
+    Ps, _ = oracle.amg_hierarchy(Am, **kw)
+    amg = U.AlgebraicMultigrid(ctx, smoother="jacobi", **{option: 1}, **kw)
+    M = U.SparseMatrix(ctx, A)
+    omg = oracle.Multigrid(Am, Ps, smoother="jacobi", fix_semidefinite=fix)
+    for _ in range(2):
+        amg.update(M)
+        for l in range(amg.n_levels()):
+            rp, ci, v = amg.level_matrix(l).csr()
+            orp, oci, ov = omg.level_matrix(l).arrays()
+            np.testing.assert_array_equal(rp, orp)
+            np.testing.assert_array_equal(ci, oci)
+            np.testing.assert_allclose(v, ov, rtol=1e-12, atol=1e-12 * np.abs(ov).max())
+
+
 def test_reference_amg_1d_case(ctx, oracle):
     """utopia/tests/utopia_AMGTest.cpp:36-110 (1D Laplacian, 100 dofs, identity boundary rows,
     b = 2 with 0 on the boundary, 6 levels, atol 1e-6, ||r||_1 < 1e-5), with Chebyshev3level

@@ -502,7 +502,10 @@ public:
         UGPU_CHECK(want_levels == 0 || want_levels >= 2, UGPU_ERR_ARG, "n_levels must be 0 (automatic) or >= 2");
         transfers_.clear();
         parents_.clear();
-        std::vector<std::unique_ptr<Mat>> products;
+        // The multigrid takes the products from here (a second time they took 2.2 ms of kernels at 95 x 89 x 97), unless
+        // it forms others: from levels whose semidefinite diagonals it has fixed, or with their structure kept.
+        const bool hand_over = get("fix_semidefinite_operators") == 0 && get("keep_galerkin_structure") == 0;
+        std::vector<std::unique_ptr<Mat>> products;  // only the last one where they are not handed over
         const Mat *cur = A;
         std::vector<int32_t> rp, ci, parent;
         std::vector<double> v, amax;
@@ -530,6 +533,7 @@ public:
             auto next = ptap(*cur, *P);  // IPRTransfer::restrict(M): P^T M P
             transfers_.push_back(std::move(P));
             cur = next.get();
+            if (!hand_over) products.clear();
             products.push_back(std::move(next));
         }
         UGPU_CHECK(!transfers_.empty(), UGPU_ERR_ARG, "algebraic multigrid: no coarse level");
@@ -537,7 +541,8 @@ public:
         std::vector<const Mat *> P;
         for (auto it = transfers_.rbegin(); it != transfers_.rend(); ++it) P.push_back(it->get());
         mg_set_transfers(mg_.get(), P);
-        mg_set_products(mg_.get(), std::move(products));  // a second time they took 2.2 ms of kernels at 95 x 89 x 97
+        if (hand_over) mg_set_products(mg_.get(), std::move(products));
+        else products.clear();
         mg_->update(A);
     }
 
