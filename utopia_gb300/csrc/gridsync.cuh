@@ -66,6 +66,7 @@ struct GridExchange {
                 }
             }
         }
+        __syncwarp();  // orders the other lanes' reads of the partials behind lane 0's acquire; a shuffle does not
         ok = __shfl_sync(0xffffffffu, ok, 0);
         unsigned long long s[NV];
 #pragma unroll
