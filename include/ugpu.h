@@ -271,6 +271,9 @@ UGPU_API int ugpu_spmv_dot(const ugpu_mat *A, const ugpu_vec *x, ugpu_vec *y, ug
  * operator does not take the staged kernel (nothing runs). */
 UGPU_API int ugpu_test_staged_wait_timeout(const ugpu_mat *A, const ugpu_vec *x, ugpu_vec *y, int64_t spin_cycles,
                                            int *launched);
+/* Test only: with on != 0 every launch of a resident solver kernel (CG, MPRGP, power method) through this context
+ * fails as on a device that does not hold its CTAs at once, until it is set back to 0. */
+UGPU_API int ugpu_test_refuse_resident(ugpu_ctx *ctx, int on);
 /* r = b - A x (Eval_Residual, utopia/utopia_core/eval/utopia_Eval_Residual.hpp:19-38), one pass */
 UGPU_API int ugpu_residual(const ugpu_mat *A, const ugpu_vec *b, const ugpu_vec *x, ugpu_vec *r);
 /* fused Jacobi sweep x_out = x + omega * d^+ (b - A x) (utopia/solvers/smoothers/utopia_Jacobi.hpp:131-141

@@ -29,6 +29,14 @@ def ctx():
     c.close()
 
 
+@pytest.fixture
+def separate_kernels(ctx):
+    """Resident solver kernels are refused, as on a device that does not hold their CTAs at once."""
+    assert ctx.lib.ugpu_test_refuse_resident(ctx.h, 1) == 0
+    yield
+    assert ctx.lib.ugpu_test_refuse_resident(ctx.h, 0) == 0
+
+
 @pytest.fixture(scope="session")
 def oracle():
     import oracle as O

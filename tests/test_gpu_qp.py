@@ -241,6 +241,33 @@ def test_mprgp_graph_and_eager_are_bitwise_equal(ctx, oracle):
     assert np.array_equal(xg == lb, xo == lb)
 
 
+@pytest.mark.parametrize("N", [40, 96])
+def test_mprgp_refused_resident_launch(ctx, oracle, separate_kernels, N):
+    """Where the device refuses the resident kernel (one cluster, a cooperative grid) the separate kernels take the
+    solve: a contact problem with a free boundary to convergence, in a graph (the expansion tail under an IF node)
+    and launched one by one (the tail gated) with the same bits, and the oracle's active set."""
+    h = 1.0 / (N + 1)
+    A, b, lb, ub = P.obstacle_qp(N, seed=3, rhs=-10.0 * h * h)
+    atol = 1e-9 * h * h
+    out = []
+    for graphs in (1, 0):
+        s = U.MPRGP(ctx, atol=atol, rtol=1e-30, max_it=100000, use_graphs=graphs)
+        vlb, vub = U.Vector(ctx, lb), U.Vector(ctx, ub)
+        s.set_box_constraints(vlb, vub)
+        x = U.Vector(ctx, n=A.nrows)
+        s.solve(U.SparseMatrix(ctx, A), U.Vector(ctx, b), x)
+        st = s.solution_status()
+        assert st["converged"] and st["kernel_launches"] >= 3 * st["iterates"]  # the separate kernels ran
+        out.append((x.numpy(), st["iterates"]))
+    assert out[0][1] == out[1][1]
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    xo, so = oracle.mprgp_solve(oracle.Matrix(A), b, lb, ub, atol=atol, rtol=1e-30, max_it=100000)
+    xg = out[0][0]
+    assert np.array_equal(xg == lb, xo == lb)
+    assert 0 < (xg == lb).sum() < A.nrows
+    assert np.linalg.norm(xg - xo) <= 1e-8 * np.linalg.norm(xo)
+
+
 def _penalty_gpu(ctx, A, b, ub=None, lb=None, selection=None, T=None, O=None, S=None, x0=None, solver=None, **prm):
     s = solver or U.ShiftedPenaltyQPSolver(ctx, **prm)
     keep = [U.Vector(ctx, v) if v is not None else None for v in (lb, ub, selection)]

@@ -86,6 +86,41 @@ def test_cg_resident_forms(ctx, oracle, shape, precond):
     assert rel(x.numpy(), xo) <= 1e-11
 
 
+@pytest.mark.parametrize("shape", [(48, 48), (61, 101), (300, 220), "graph4001"])
+@pytest.mark.parametrize("precond", ["invdiag", "none"])
+def test_cg_refused_resident_launch(ctx, oracle, separate_kernels, shape, precond):
+    """Where the device refuses the resident kernel (as one cluster or as a cooperative grid) the separate kernels
+    take the solve: in a graph and launched one by one the same bits, and the oracle's iterations to convergence."""
+    A = P.laplacian_2d(*shape) if isinstance(shape, tuple) else P.random_spd_graph(int(shape[5:]), 4, 1)
+    b = np.random.default_rng(A.nrows).uniform(-1.0, 1.0, A.nrows)
+    atol = 1e-8 * np.linalg.norm(b)
+    xo, so = oracle.cg_solve(oracle.Matrix(A), b, precond=precond, atol=atol)
+    out = []
+    for graphs in (1, 0):
+        s = cg(ctx, U.InvDiagPreconditioner(ctx) if precond == "invdiag" else None, atol=atol, use_graphs=graphs)
+        x = U.Vector(ctx, n=A.nrows)
+        assert s.solve(U.SparseMatrix(ctx, A), U.Vector(ctx, b), x)
+        st = s.solution_status()
+        assert st["kernel_launches"] >= 3 * st["iterates"]  # the separate kernels ran
+        assert abs(st["iterates"] - so["iterates"]) <= 1
+        assert np.linalg.norm(b - A.matvec(x.numpy())) <= atol * 1.001
+        out.append((x.numpy(), st["iterates"]))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    assert out[0][1] == out[1][1]
+
+
+def test_power_method_refused_resident_launch(ctx, oracle, separate_kernels):
+    A = P.laplacian_2d(192)
+    Ps = P.hierarchy_2d(192, 4)
+    omg = oracle.Multigrid(oracle.Matrix(A), Ps, smoother="chebyshev")
+    mg = U.Multigrid(ctx, smoother="chebyshev")
+    mg.set_transfer_operators(Ps)
+    M = U.SparseMatrix(ctx, A)
+    mg.update(M)
+    for l in range(1, 4):
+        np.testing.assert_allclose(mg.eigs(l), omg.eigs(l), rtol=1e-12)
+
+
 def test_cg_max_it_and_initial_guess(ctx, oracle):
     A, b = P.poisson2d_cg(32, 1)
     x0 = np.random.default_rng(3).standard_normal(A.nrows)

@@ -401,12 +401,13 @@ public:
         if (mode_ != CG_GENERIC && !flexible_ && CgResident::fits(*ctx, *op)) {
             if (!sums_.ptr) sums_.alloc(CgResident::sum_bytes(*ctx));
             const double *dinv = mode_ == CG_JACOBI ? static_cast<InvDiag *>(pc_)->d.as<double>() : nullptr;
-            CgResident::run(*ctx, *op, b.as<double>(), x.as<double>(), dinv, z_.as<double>(), p_.as<double>(),
-                            Ap_.as<double>(), sums_.ptr, dev_.as<CgDev>(), get("atol"), (long long)get("max_it"));
-            UGPU_CUDA(cudaMemcpyAsync(host_dev_, dev_.ptr, sizeof(CgDev), cudaMemcpyDeviceToHost, ctx->stream));
-            ctx->check_kernel_flags();
-            finish(t0, l0, false, 0);
-            return;
+            if (CgResident::run(*ctx, *op, b.as<double>(), x.as<double>(), dinv, z_.as<double>(), p_.as<double>(),
+                                Ap_.as<double>(), sums_.ptr, dev_.as<CgDev>(), get("atol"), (long long)get("max_it"))) {
+                UGPU_CUDA(cudaMemcpyAsync(host_dev_, dev_.ptr, sizeof(CgDev), cudaMemcpyDeviceToHost, ctx->stream));
+                ctx->check_kernel_flags();
+                finish(t0, l0, false, 0);
+                return;
+            }
         }
         // r = b - A x
         {

@@ -23,9 +23,10 @@ struct CgDev {
 // A whole solve of small systems (unpreconditioned, or Jacobi with the weights dinv) as one cooperative kernel
 struct CgResident {
     static bool fits(const Context &c, const Mat &A);
-    // dev receives the final state; z, p0, p1: n doubles each; sums: sum_bytes(); work on c.stream
+    // dev receives the final state; z, p0, p1: n doubles each; sums: sum_bytes(); work on c.stream.  False: the device
+    // does not hold the kernel's CTAs at once, x is as it was
     static size_t sum_bytes(const Context &c);
-    static void run(Context &c, const Mat &A, const double *b, double *x, const double *dinv, double *z, double *p0,
+    static bool run(Context &c, const Mat &A, const double *b, double *x, const double *dinv, double *z, double *p0,
                     double *p1, void *sums, CgDev *dev, double atol, long long max_it);
 };
 

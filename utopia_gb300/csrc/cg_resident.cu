@@ -340,7 +340,7 @@ bool CgResident::fits(const Context &c, const Mat &A) {
 
 size_t CgResident::sum_bytes(const Context &c) { return 2 * GridExchange<1>::bytes(c.sms); }
 
-void CgResident::run(Context &c, const Mat &A, const double *b, double *x, const double *dinv, double *z, double *p0,
+bool CgResident::run(Context &c, const Mat &A, const double *b, double *x, const double *dinv, double *z, double *p0,
                      double *p1, void *sums, CgDev *dev, double atol, long long max_it) {
     const int64_t n = A.nrows;
     // One cluster of 16 CTAs up to kClusterRows rows; otherwise a CTA per SM.  At least 64 rows per CTA: below that
@@ -377,7 +377,7 @@ void CgResident::run(Context &c, const Mat &A, const double *b, double *x, const
                          : rpt == 1 ? (reg ? k_cg_resident<1, true, false> : k_cg_resident<1, false, false>)
                          : rpt == 2 ? (reg ? k_cg_resident<2, true, false> : k_cg_resident<2, false, false>)
                                     : k_cg_resident<4, false, false>;
-    launch_resident(c, f, a, int(G), nt, smem, cl);
+    return launch_resident(c, f, a, int(G), nt, smem, cl);
 }
 
 }  // namespace ugpu

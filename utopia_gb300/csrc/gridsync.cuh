@@ -200,9 +200,11 @@ __device__ __forceinline__ double warp_sum_of(const double *sh, int n) {
     return s;
 }
 
-// Launches a resident kernel: as one cluster (of at most 16 CTAs), or cooperatively.
+// Launches a resident kernel: as one cluster (of at most 16 CTAs), or cooperatively.  False where the device will not
+// hold all its CTAs at once (a process with a share of the SMs, for example): nothing has run, and the
+// separate kernels take the solve.  The launch itself says so; an occupancy query before each would cost time.
 template <class Args>
-inline void launch_resident(Context &c, void (*kernel)(Args), const Args &args, int ctas, int threads, size_t smem,
+inline bool launch_resident(Context &c, void (*kernel)(Args), const Args &args, int ctas, int threads, size_t smem,
                             bool cluster) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(ctas));
@@ -210,8 +212,9 @@ inline void launch_resident(Context &c, void (*kernel)(Args), const Args &args, 
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
     cudaLaunchAttribute at[1];
+    cudaError_t e = cudaSuccess;
     if (cluster) {
-        UGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = unsigned(ctas);
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -221,8 +224,20 @@ inline void launch_resident(Context &c, void (*kernel)(Args), const Args &args, 
     }
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    UGPU_CUDA(cudaLaunchKernelEx(&cfg, kernel, args));
+    if (c.refuse_resident) e = cluster ? cudaErrorInvalidClusterSize : cudaErrorCooperativeLaunchTooLarge;
+    else if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kernel, args);
+    switch (e) {
+    case cudaErrorCooperativeLaunchTooLarge:
+    case cudaErrorInvalidClusterSize:
+    case cudaErrorLaunchOutOfResources:
+    case cudaErrorInvalidConfiguration:
+    case cudaErrorNotSupported:
+        cudaGetLastError();
+        return false;
+    default: UGPU_CUDA(e);
+    }
     c.launches++;
+    return true;
 }
 
 }  // namespace ugpu

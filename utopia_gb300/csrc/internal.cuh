@@ -161,6 +161,7 @@ struct Context {
     Buffer kflags;     // int[4] device error flags; [0]: a staged SpMV gave up waiting for its copies; [1]: a
                        // dense product gave up waiting for its MMAs; [2]: a resident kernel gave up waiting for its CTAs
     long long staged_test_spin = 0;  // > 0 only inside ugpu_test_staged_wait_timeout
+    bool refuse_resident = false;    // set by ugpu_test_refuse_resident alone
     double *host_scalars = nullptr;  // pinned mirror
     int64_t launches = 0;            // kernels launched through this context (instrumentation)
     Context(int dev);

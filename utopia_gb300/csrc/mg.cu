@@ -707,11 +707,10 @@ private:
         for (int l = 1; l < L; ++l) {
             const Level &lv = levels_[l];
             if (!pm_resident_fits(*ctx, *lv.A64)) continue;
-            resident[l] = 1;
             PmScratch &ps = pm_[l];
             ps.sums.ensure(pm_resident_bytes(*ctx));
-            pm_resident(*ctx, *lv.A64, ps.v.as<double>(), ps.w.as<double>(), ps.sums.ptr, ps.st.as<double>() + 1, tol,
-                        max_it);
+            resident[l] = pm_resident(*ctx, *lv.A64, ps.v.as<double>(), ps.w.as<double>(), ps.sums.ptr,
+                                      ps.st.as<double>() + 1, tol, max_it);
         }
         UGPU_CUDA(cudaEventRecord(pm_fork_, main));
         for (int l = 1; l < L; ++l) {

@@ -18,14 +18,15 @@ struct QpDev {
 };
 
 // A solve of small problems as one kernel (work on c.stream).
-// fi, beta, p0, p1: n doubles each; sums: sum_bytes(); dev receives the final state.
+// fi, beta, p0, p1: n doubles each; sums: sum_bytes(); dev receives the final state.  False from run(): the
+// device does not hold the kernel's CTAs at once, x is as it was.
 struct MprgpResident {
     static bool fits(const Context &c, const Mat &A);
     // Whether run() makes the power-method estimate itself (lambda = 0): up to two rows per thread.  On larger
     // problems its 0.6 ms of host round trips is nothing beside the solve.
     static bool own_power_method(const Context &c, const Mat &A);
     static size_t sum_bytes(const Context &c);
-    static void run(Context &c, const Mat &A, const double *b, double *x, const double *lb, const double *ub, double *fi,
+    static bool run(Context &c, const Mat &A, const double *b, double *x, const double *lb, const double *ub, double *fi,
                     double *beta, double *p0, double *p1, void *sums, QpDev *dev, double atol, double rtol,
                     long long max_it, double lambda, double eig_tol, long long eig_max_it);
 };

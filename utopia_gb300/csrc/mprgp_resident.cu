@@ -561,7 +561,7 @@ size_t MprgpResident::sum_bytes(const Context &c) {
     return GridExchange<3, 4>::bytes(c.sms) + GridExchange<4>::bytes(c.sms);
 }
 
-void MprgpResident::run(Context &c, const Mat &A, const double *b, double *x, const double *lb, const double *ub,
+bool MprgpResident::run(Context &c, const Mat &A, const double *b, double *x, const double *lb, const double *ub,
                         double *fi, double *beta, double *p0, double *p1, void *sums, QpDev *dev, double atol,
                         double rtol, long long max_it, double lambda, double eig_tol, long long eig_max_it) {
     const int64_t n = A.nrows;
@@ -605,7 +605,7 @@ void MprgpResident::run(Context &c, const Mat &A, const double *b, double *x, co
                            : rpt == 1 ? (reg ? k_mprgp_resident<1, true, false> : k_mprgp_resident<1, false, false>)
                            : rpt == 2 ? (reg ? k_mprgp_resident<2, true, false> : k_mprgp_resident<2, false, false>)
                                       : k_mprgp_resident<4, false, false>;
-    launch_resident(c, f, a, int(G), nt, smem, cl);
+    return launch_resident(c, f, a, int(G), nt, smem, cl);
 }
 
 }  // namespace ugpu

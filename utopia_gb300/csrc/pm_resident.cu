@@ -169,7 +169,7 @@ bool pm_resident_fits(const Context &c, const Mat &A) {
 
 size_t pm_resident_bytes(const Context &c) { return GridExchange<1>::bytes(c.sms); }
 
-void pm_resident(Context &c, const Mat &A, double *y0, double *y1, void *sums, double *lambda, double tol,
+bool pm_resident(Context &c, const Mat &A, double *y0, double *y1, void *sums, double *lambda, double tol,
                  long long max_it) {
     const int64_t n = A.nrows;
     const bool reg = A.max_row <= kRegRow, cl = reg && n <= kClusterRows;
@@ -196,7 +196,7 @@ void pm_resident(Context &c, const Mat &A, double *y0, double *y1, void *sums, d
     void (*f)(PmArgs) = cl         ? k_pm_resident<1, true, true>
                         : rpt == 1 ? (reg ? k_pm_resident<1, true, false> : k_pm_resident<1, false, false>)
                                    : (reg ? k_pm_resident<2, true, false> : k_pm_resident<2, false, false>);
-    launch_resident(c, f, a, int(G), nt, smem, cl);
+    return launch_resident(c, f, a, int(G), nt, smem, cl);
 }
 
 }  // namespace ugpu

@@ -605,15 +605,16 @@ public:
         if (MprgpResident::fits(*ctx, *op)) {
             if (!sums_.ptr) sums_.alloc(MprgpResident::sum_bytes(*ctx));
             const double lambda = MprgpResident::own_power_method(*ctx, *op) ? 0.0 : power_method();
-            MprgpResident::run(*ctx, *op, rhs.as<double>(), x.as<double>(), lb, ub, fi_.as<double>(),
-                               beta_.as<double>(), p_.as<double>(), Ap_.as<double>(), sums_.ptr, dev_.as<QpDev>(),
-                               get("atol"), get("rtol"), (long long)get("max_it"), lambda, get("eig_comp_tol"),
-                               (long long)get("power_method_max_it"));
-            UGPU_CUDA(cudaMemcpyAsync(host_, dev_.ptr, sizeof(QpDev), cudaMemcpyDeviceToHost, ctx->stream));
-            ctx->check_kernel_flags();
-            prm["lambda_max"] = lambda_max = host_->lambda;
-            finish(t0, l0);
-            return;
+            if (MprgpResident::run(*ctx, *op, rhs.as<double>(), x.as<double>(), lb, ub, fi_.as<double>(),
+                                   beta_.as<double>(), p_.as<double>(), Ap_.as<double>(), sums_.ptr, dev_.as<QpDev>(),
+                                   get("atol"), get("rtol"), (long long)get("max_it"), lambda, get("eig_comp_tol"),
+                                   (long long)get("power_method_max_it"))) {
+                UGPU_CUDA(cudaMemcpyAsync(host_, dev_.ptr, sizeof(QpDev), cudaMemcpyDeviceToHost, ctx->stream));
+                ctx->check_kernel_flags();
+                prm["lambda_max"] = lambda_max = host_->lambda;
+                finish(t0, l0);
+                return;
+            }
         }
         lambda_max = power_method();
         prm["lambda_max"] = lambda_max;

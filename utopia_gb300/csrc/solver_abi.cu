@@ -150,6 +150,13 @@ int ugpu_mg_vcycle(ugpu_solver *mg, const ugpu_vec *r, ugpu_vec *z) {
     UGPU_ABI_END(mg ? mg->impl->ctx : nullptr)
 }
 
+int ugpu_test_refuse_resident(ugpu_ctx *ctx, int on) {
+    UGPU_ABI_BEGIN
+    UGPU_REQUIRE(ctx);
+    ctx->impl.refuse_resident = on != 0;
+    UGPU_ABI_END(ctx ? &ctx->impl : nullptr)
+}
+
 int ugpu_solver_update(ugpu_solver *s, const ugpu_mat *A) {
     UGPU_ABI_BEGIN
     UGPU_REQUIRE(s);
