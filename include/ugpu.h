@@ -274,6 +274,11 @@ UGPU_API int ugpu_test_staged_wait_timeout(const ugpu_mat *A, const ugpu_vec *x,
 /* Test only: with on != 0 every launch of a resident solver kernel (CG, MPRGP, power method) through this context
  * fails as on a device that does not hold its CTAs at once, until it is set back to 0. */
 UGPU_API int ugpu_test_refuse_resident(ugpu_ctx *ctx, int on);
+/* Test only, failure detection without a GPU fault, as ugpu_test_staged_wait_timeout: a split FP64 product on the tensor
+ * cores whose first stage never reports its end; an exchange between the CTAs of a resident kernel (a cluster's
+ * or a cooperative grid's) in which one does not take part.  The wait runs out after spin_cycles. */
+UGPU_API int ugpu_test_product_wait_timeout(ugpu_ctx *ctx, int64_t spin_cycles);
+UGPU_API int ugpu_test_exchange_wait_timeout(ugpu_ctx *ctx, int cluster, int64_t spin_cycles);
 /* r = b - A x (Eval_Residual, utopia/utopia_core/eval/utopia_Eval_Residual.hpp:19-38), one pass */
 UGPU_API int ugpu_residual(const ugpu_mat *A, const ugpu_vec *b, const ugpu_vec *x, ugpu_vec *r);
 /* fused Jacobi sweep x_out = x + omega * d^+ (b - A x) (utopia/solvers/smoothers/utopia_Jacobi.hpp:131-141

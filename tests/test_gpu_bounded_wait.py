@@ -37,3 +37,31 @@ def test_staged_wait_runs_out_and_the_context_stays_usable(ctx, dtype):
     vals = M.csr()[2]
     ref = P.CSR(A.nrows, A.ncols, A.rowptr, A.colidx, vals).matvec(xh.astype(np.float64))
     np.testing.assert_allclose(y.numpy(), ref, rtol=2e-5, atol=2e-5 * np.abs(ref).max())
+
+
+def _times_out_once(ctx, rc, message):
+    lib = ctx.lib
+    assert rc == 0, lib.ugpu_last_error(ctx.h)
+    assert lib.ugpu_synchronize(ctx.h) < 0
+    assert message in lib.ugpu_last_error(ctx.h)
+    assert lib.ugpu_synchronize(ctx.h) == 0  # the flag was cleared
+
+
+def test_product_wait_runs_out_and_the_context_stays_usable(ctx):
+    """The split products of the dense factorisation: the tensor memory is given back and the next ones are right."""
+    _times_out_once(ctx, ctx.lib.ugpu_test_product_wait_timeout(ctx.h, 2_000_000), b"dense product timed out")
+    A, b = P.poisson2d_cg(32, 0)  # 1024 rows
+    x = U.Vector(ctx, n=A.nrows)
+    U.CholeskySolver(ctx).solve(U.SparseMatrix(ctx, A), U.Vector(ctx, b), x)
+    assert np.linalg.norm(b - A.matvec(x.numpy())) <= 1e-12 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("cluster", [0, 1])
+def test_exchange_wait_runs_out_and_the_context_stays_usable(ctx, cluster):
+    _times_out_once(ctx, ctx.lib.ugpu_test_exchange_wait_timeout(ctx.h, cluster, 2_000_000), b"timed out waiting for its other")
+    A, b = P.poisson2d_cg(48 if cluster else 100, 0)
+    atol = 1e-8 * np.linalg.norm(b)
+    s = U.ConjugateGradient(ctx, atol=atol)
+    x = U.Vector(ctx, n=A.nrows)
+    assert s.solve(U.SparseMatrix(ctx, A), U.Vector(ctx, b), x)
+    assert np.linalg.norm(b - A.matvec(x.numpy())) <= atol * 1.001

@@ -47,7 +47,7 @@ constexpr int kScanInside = 128;                   // K up to which a tile finds
 
 __device__ __forceinline__ uint32_t saddr(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
-__device__ __forceinline__ bool mma_wait(uint64_t *bar, uint32_t parity) {
+__device__ __forceinline__ bool mma_wait(uint64_t *bar, uint32_t parity, long long limit) {
     const long long t0 = clock64();
     while (true) {
         uint32_t ok;
@@ -59,7 +59,7 @@ __device__ __forceinline__ bool mma_wait(uint64_t *bar, uint32_t parity) {
             : "r"(saddr(bar)), "r"(parity)
             : "memory");
         if (ok) return true;
-        if (clock64() - t0 > kSpin) return false;
+        if (clock64() - t0 > limit) return false;
     }
 }
 
@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm64(const Gemm64 g, const ui
                     mma_f16(tmem + uint32_t((s + h) * GN), da + uint64_t((s * kSliceA + q * 256) >> 4),
                             db + uint64_t((h * kSliceB + q * 256) >> 4), instr_desc(n), (s | q) ? 1u : cont);
                 }
+        if (g.lose_commit && c == 0) return;
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                          saddr(&bar[c & 1]))
                      : "memory");
@@ -372,11 +373,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm64(const Gemm64 g, const ui
     int late = 0;
     for (int c = 0; c < nk; ++c) {
         // the stage's last MMAs (two stages ago) must have read it
-        if (c >= 2 && !mma_wait(&bar[c & 1], uint32_t((c >> 1) - 1) & 1u)) late = 1;
+        if (c >= 2 && !mma_wait(&bar[c & 1], uint32_t((c >> 1) - 1) & 1u, g.spin)) late = 1;
         split(c);
         if (c + 1 < nk) load(c + 1);
         if (c > 0 && c % kFlush == 0) {
-            if (!mma_wait(&bar[(c - 1) & 1], uint32_t((c - 1) >> 1) & 1u)) late = 1;
+            if (!mma_wait(&bar[(c - 1) & 1], uint32_t((c - 1) >> 1) & 1u, g.spin)) late = 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             flush();
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm64(const Gemm64 g, const ui
         }
     }
     if (nk > 0 && !late) {
-        if (!mma_wait(&bar[(nk - 1) & 1], uint32_t((nk - 1) >> 1) & 1u)) late = 1;
+        if (!mma_wait(&bar[(nk - 1) & 1], uint32_t((nk - 1) >> 1) & 1u, g.spin)) late = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         flush();
     }
@@ -560,6 +561,8 @@ void gemm64(Context &c, const Gemm64 &args, Buffer &scales) {
         UGPU_LAUNCH_CHECK();
         return;
     }
+    g.spin = c.product_test_spin > 0 ? c.product_test_spin : kSpin;
+    g.lose_commit = c.product_test_spin > 0;
     uint32_t *eA = nullptr, *eB = nullptr;
     if (g.K > kScanInside) {
         scales.ensure(sizeof(uint32_t) * (size_t(g.M) + size_t(g.N)));
@@ -584,3 +587,31 @@ void gemm64(Context &c, const Gemm64 &args, Buffer &scales) {
 }
 
 }  // namespace ugpu
+
+using namespace ugpu;
+
+extern "C" int ugpu_test_product_wait_timeout(ugpu_ctx *ctx, int64_t spin_cycles) {
+    UGPU_ABI_BEGIN
+    UGPU_REQUIRE(ctx);
+    UGPU_CHECK(spin_cycles > 0 && spin_cycles <= 100000000ll, UGPU_ERR_ARG, "test wait limit: 1 .. 1e8 cycles");
+    Context &c = ctx->impl;
+    Buffer operands, out, scales;
+    operands.alloc(sizeof(double) * 512 * 512);
+    out.alloc(sizeof(double) * 512 * 512);
+    UGPU_CUDA(cudaMemsetAsync(operands.ptr, 0, operands.bytes, c.stream));
+    Gemm64 g;
+    g.M = g.N = g.K = 512;
+    g.A = g.B = operands.as<double>();
+    g.a_row = g.b_row = 512;
+    g.a_k = g.b_k = 1;
+    g.C = out.as<double>();
+    g.ldc = 512;
+    struct Reset {
+        Context &c;
+        ~Reset() { c.product_test_spin = 0; }
+    } reset{c};
+    c.product_test_spin = spin_cycles;
+    gemm64(c, g, scales);
+    cudaStreamSynchronize(c.stream);  // before the buffers go
+    UGPU_ABI_END(ctx ? &ctx->impl : nullptr)
+}

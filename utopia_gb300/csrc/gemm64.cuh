@@ -27,6 +27,8 @@ struct Gemm64 {
     int flags = 0;
     bool fma = false;  // FP64 multiply-adds throughout: no split product
     int vec_a = 0, vec_b = 0;  // set by gemm64()
+    long long spin = 0;        // likewise: clock cycles that a wait may take
+    bool lose_commit = false;  // likewise, in a test: the first stage's MMAs never report their end
 };
 // scales: scratch of at least M + N 32-bit words, grown where it is smaller (stream-ordered use)
 void gemm64(Context &c, const Gemm64 &g, Buffer &scales);

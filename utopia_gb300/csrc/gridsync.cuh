@@ -38,6 +38,7 @@ struct GridExchange {
     using V = Values<NV, MIN>;
     unsigned long long *count, *part;  // part: [2][NV][G]
     int G;                             // CTAs
+    long long limit = kGridSpin;
     static constexpr size_t bytes(int G) { return 128 + sizeof(unsigned long long) * 2 * NV * size_t(G); }
     __device__ __forceinline__ void init(char *base, int ctas) {
         count = reinterpret_cast<unsigned long long *>(base);
@@ -60,7 +61,7 @@ struct GridExchange {
             while (true) {
                 asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(have) : "l"(count) : "memory");
                 if (have >= want) break;
-                if (clock64() - t0 > kGridSpin) {
+                if (clock64() - t0 > limit) {
                     ok = 0;
                     break;
                 }
@@ -107,6 +108,7 @@ struct ClusterExchange {
     using V = Values<NV, MIN>;
     uint32_t slots, bars;  // shared addresses: [2][NV][16] 64-bit slots, [2] mbarriers
     uint32_t rank, size;
+    long long limit = kGridSpin;
     static constexpr int kDoubles = 2 * NV * 16 + 2;  // shared 8-byte words
     __device__ __forceinline__ void init(double *shared, uint32_t r, uint32_t n) {
         slots = uint32_t(__cvta_generic_to_shared(shared));
@@ -145,7 +147,7 @@ struct ClusterExchange {
                 : "=r"(ok)
                 : "r"(bars + 8 * b), "r"(parity)
                 : "memory");
-            if (ok || clock64() - t0 > kGridSpin) break;
+            if (ok || clock64() - t0 > limit) break;
         }
         unsigned long long s[NV];
 #pragma unroll

@@ -162,6 +162,7 @@ struct Context {
                        // dense product gave up waiting for its MMAs; [2]: a resident kernel gave up waiting for its CTAs
     long long staged_test_spin = 0;  // > 0 only inside ugpu_test_staged_wait_timeout
     bool refuse_resident = false;    // set by ugpu_test_refuse_resident alone
+    long long product_test_spin = 0; // > 0 only inside ugpu_test_product_wait_timeout
     double *host_scalars = nullptr;  // pinned mirror
     int64_t launches = 0;            // kernels launched through this context (instrumentation)
     Context(int dev);

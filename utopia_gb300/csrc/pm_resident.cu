@@ -160,6 +160,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_pm_resident(PmArgs a) {
     if (CL) cluster_barrier();  // no CTA leaves while another may still read its shared memory
 }
 
+// An exchange whose other CTA never takes part (it waits at the cluster's barrier, or there is none): the wait runs out
+template <bool CL>
+__global__ void __launch_bounds__(32) k_lonely_exchange(char *sums, long long limit, int *kflag) {
+    __shared__ double sh[ClusterExchange<1>::kDoubles];
+    __shared__ unsigned long long part[1];
+    using Exchange = typename std::conditional<CL, ClusterExchange<1>, GridExchange<1>>::type;
+    Exchange gx;
+    if constexpr (CL) {
+        gx.init(sh, blockIdx.x, gridDim.x);
+        if (threadIdx.x == 0) gx.init_barriers();
+        __syncthreads();
+        cluster_barrier();
+    } else {
+        gx.init(sums, 2);
+    }
+    gx.limit = limit;
+    if (threadIdx.x == 0) part[0] = 0;
+    __syncwarp();
+    unsigned long long out[1];
+    if (blockIdx.x == 0 && !gx.exchange(0, part, out) && threadIdx.x == 0) atomicExch(kflag, 1);
+    if (CL) cluster_barrier();
+}
+
 }  // namespace
 
 // Up to two rows per thread (155,648 rows) of at most 32 entries
@@ -200,3 +223,33 @@ bool pm_resident(Context &c, const Mat &A, double *y0, double *y1, void *sums, d
 }
 
 }  // namespace ugpu
+
+using namespace ugpu;
+
+extern "C" int ugpu_test_exchange_wait_timeout(ugpu_ctx *ctx, int cluster, int64_t spin_cycles) {
+    UGPU_ABI_BEGIN
+    UGPU_REQUIRE(ctx);
+    UGPU_CHECK(spin_cycles > 0 && spin_cycles <= 100000000ll, UGPU_ERR_ARG, "test wait limit: 1 .. 1e8 cycles");
+    Context &c = ctx->impl;
+    Buffer sums;
+    sums.alloc(GridExchange<1>::bytes(2));
+    UGPU_CUDA(cudaMemsetAsync(sums.ptr, 0, sums.bytes, c.stream));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster ? 2 : 1);
+    cfg.blockDim = dim3(32);
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cfg.gridDim.x;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    char *p = static_cast<char *>(sums.ptr);
+    const long long limit = spin_cycles;
+    int *flag = c.d_kflags() + 2;
+    if (cluster) UGPU_CUDA(cudaLaunchKernelEx(&cfg, k_lonely_exchange<true>, p, limit, flag));
+    else UGPU_CUDA(cudaLaunchKernelEx(&cfg, k_lonely_exchange<false>, p, limit, flag));
+    c.launches++;
+    cudaStreamSynchronize(c.stream);  // before the buffer goes
+    UGPU_ABI_END(ctx ? &ctx->impl : nullptr)
+}
