@@ -279,6 +279,9 @@ UGPU_API int ugpu_test_refuse_resident(ugpu_ctx *ctx, int on);
  * or a cooperative grid's) in which one does not take part.  The wait runs out after spin_cycles. */
 UGPU_API int ugpu_test_product_wait_timeout(ugpu_ctx *ctx, int64_t spin_cycles);
 UGPU_API int ugpu_test_exchange_wait_timeout(ugpu_ctx *ctx, int cluster, int64_t spin_cycles);
+/* Test only: the calling thread's next cudaMalloc of this library fails as on a full device; the allocation then gives the
+ * memory pool's unused part back and is tried once more. */
+UGPU_API int ugpu_test_fail_allocation(void);
 /* r = b - A x (Eval_Residual, utopia/utopia_core/eval/utopia_Eval_Residual.hpp:19-38), one pass */
 UGPU_API int ugpu_residual(const ugpu_mat *A, const ugpu_vec *b, const ugpu_vec *x, ugpu_vec *r);
 /* fused Jacobi sweep x_out = x + omega * d^+ (b - A x) (utopia/solvers/smoothers/utopia_Jacobi.hpp:131-141

@@ -65,3 +65,21 @@ def test_exchange_wait_runs_out_and_the_context_stays_usable(ctx, cluster):
     x = U.Vector(ctx, n=A.nrows)
     assert s.solve(U.SparseMatrix(ctx, A), U.Vector(ctx, b), x)
     assert np.linalg.norm(b - A.matvec(x.numpy())) <= atol * 1.001
+
+
+def test_full_device_gives_the_pool_back(ctx):
+    """A vector that finds no memory gets what finished set-ups left in the pool."""
+    import torch
+
+    A, Ps, _ = P.poisson3d_mg(64, 3, seed=1)
+    mg = U.Multigrid(ctx, smoother="jacobi")
+    mg.set_transfer_operators(Ps)
+    mg.update(U.SparseMatrix(ctx, A))
+    del mg
+    ctx.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    assert ctx.lib.ugpu_test_fail_allocation() == 0
+    v = np.random.default_rng(0).standard_normal(1000)
+    x = U.Vector(ctx, v)
+    np.testing.assert_array_equal(x.numpy(), v)
+    assert torch.cuda.mem_get_info()[0] > before + (8 << 20)  # the hierarchy's 262,144 x 7 entries alone are 22 MB

@@ -83,6 +83,7 @@ SIGNATURES = {
     "ugpu_active_set_compact": [_vp, _vp, _vp, _i32, _vp, C.POINTER(_i64)],
     "ugpu_test_staged_wait_timeout": [_vp, _vp, _vp, _i64, C.POINTER(_int)],
     "ugpu_test_refuse_resident": [_vp, _int],
+    "ugpu_test_fail_allocation": [],
     "ugpu_test_product_wait_timeout": [_vp, _i64],
     "ugpu_test_exchange_wait_timeout": [_vp, _int, _i64],
     "ugpu_dots_noalloc": [_int, _pp, _pp, C.POINTER(_int), C.POINTER(_int), _i64, _vp, _vp],

@@ -14,10 +14,10 @@ thread_local const std::shared_ptr<StreamRef> *PoolScope::current = nullptr;
 
 // The device's pool (one per process): keeps at most a sixteenth of the device's memory beyond what is in use, the
 // size of a 192^3 hierarchy several times over.  Null where the device has none: plain allocations then.
+static std::mutex pools_mutex;
+static std::map<int, cudaMemPool_t> pools;
 static cudaMemPool_t device_pool(int dev, size_t memory) {
-    static std::mutex mutex;
-    static std::map<int, cudaMemPool_t> pools;
-    std::lock_guard<std::mutex> lock(mutex);
+    std::lock_guard<std::mutex> lock(pools_mutex);
     auto it = pools.find(dev);
     if (it != pools.end()) return it->second;
     int supported = 0;
@@ -34,6 +34,24 @@ static cudaMemPool_t device_pool(int dev, size_t memory) {
     }
     pools[dev] = pool;
     return pool;
+}
+
+void trim_device_pool() {
+    int dev = 0;
+    UGPU_CUDA(cudaGetDevice(&dev));
+    UGPU_CUDA(cudaDeviceSynchronize());
+    std::lock_guard<std::mutex> lock(pools_mutex);
+    auto it = pools.find(dev);
+    if (it != pools.end() && it->second) UGPU_CUDA(cudaMemPoolTrimTo(it->second, 0));
+}
+
+static thread_local bool fail_next_allocation = false;
+cudaError_t plain_alloc(void **ptr, size_t bytes) {
+    if (fail_next_allocation) {
+        fail_next_allocation = false;
+        return cudaErrorMemoryAllocation;
+    }
+    return cudaMalloc(ptr, bytes);
 }
 
 Context::Context(int dev) : device(dev) {
@@ -750,6 +768,11 @@ double *noalloc_scratch() {
 }
 
 }  // namespace
+
+extern "C" int ugpu_test_fail_allocation(void) {
+    ugpu::fail_next_allocation = true;
+    return 0;
+}
 
 extern "C" int ugpu_dots_noalloc(int k, const void *const *a, const void *const *b, const int *dtype_a,
                                  const int *dtype_b, int64_t n, double *d_out, void *stream) {

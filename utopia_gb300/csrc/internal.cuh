@@ -74,6 +74,10 @@ struct PoolScope {
     PoolScope(const PoolScope &) = delete;
     PoolScope &operator=(const PoolScope &) = delete;
 };
+// cudaMalloc; fails once after ugpu_test_fail_allocation
+cudaError_t plain_alloc(void **ptr, size_t bytes);
+// gives the unused memory of the current device's pool back, after the work that may still use it
+void trim_device_pool();
 struct Buffer {
     void *ptr = nullptr;
     size_t bytes = 0;
@@ -115,7 +119,13 @@ struct Buffer {
             UGPU_CUDA(e);
             ordered = r;
         } else {
-            UGPU_CUDA(cudaMalloc(&ptr, b));
+            cudaError_t e = plain_alloc(&ptr, b);
+            if (e == cudaErrorMemoryAllocation) {  // what the device's pool keeps unused, then once more
+                cudaGetLastError();
+                trim_device_pool();
+                e = plain_alloc(&ptr, b);
+            }
+            UGPU_CUDA(e);
         }
         bytes = b;
         owned = true;
