@@ -171,3 +171,25 @@ def test_aggregates_of_large_levels(ctx, oracle, name, additive, excluded):
     got, nc = amg.parent(0)
     assert nc == Pm.ncols
     np.testing.assert_array_equal(got, ref)
+
+
+def test_aggregates_of_a_long_row(ctx, oracle):
+    """One row of an arrow matrix touches every other one: the sequential aggregation takes it."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(2)
+    n = 20001
+    A = sp.diags([rng.uniform(-1, 0, n - 1), rng.uniform(5, 9, n), rng.uniform(-1, 0, n - 1)], [-1, 0, 1]).tolil()
+    A[0, 1:] = rng.uniform(-1, 0, n - 1)
+    A[1:, 0] = rng.uniform(-1, 0, n - 1).reshape(-1, 1)
+    A[0, 0] = 5.0 * n
+    Ac = P.CSR.from_scipy(A.tocsr())
+    ref, Pm = oracle.agglomerate(oracle.Matrix(Ac))
+    amg = U.AlgebraicMultigrid(ctx, smoother="jacobi", n_levels=2)
+    try:
+        amg.update(U.SparseMatrix(ctx, Ac))
+    except U.UgpuError as e:
+        assert "coarse operator" in str(e) or "coarse solver" in str(e)
+    got, nc = amg.parent(0)
+    assert nc == Pm.ncols
+    np.testing.assert_array_equal(got, ref)

@@ -90,7 +90,6 @@ struct AggState {
     unsigned int unfit;     // columns not ascending, no diagonal, or a pattern that is not symmetric
     unsigned int excluded;  // some row is excluded
     unsigned int left;      // rows whose turn has not come
-    int max_row;
 };
 
 // the word at p if `want`; a predicate and no branch, so that a row's loads are in flight together
@@ -111,7 +110,6 @@ __device__ __forceinline__ unsigned long long agg_word(int turns, int parent) {
 __global__ void __launch_bounds__(kBlock) k_agg_prepare(const int32_t *rp, const int32_t *ci, const double *v, int64_t n,
                                                         bool additive, double *a_max, unsigned long long *word,
                                                         AggState *st) {
-    int longest = 0;
     bool unfit = false, excluded = false;
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         const int32_t k0 = rp[i], k1 = rp[i + 1];
@@ -128,15 +126,12 @@ __global__ void __launch_bounds__(kBlock) k_agg_prepare(const int32_t *rp, const
         }
         unfit |= !diag && !out;
         excluded |= out;
-        longest = max(longest, k1 - k0);
         a_max[i] = m;
         word[i] = agg_word(0, out ? -2 : -1);
     }
-    longest = __reduce_max_sync(0xffffffffu, longest);
     unfit = __any_sync(0xffffffffu, unfit);
     excluded = __any_sync(0xffffffffu, excluded);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(&st->max_row, longest);
         if (unfit) atomicOr(&st->unfit, 1u);
         if (excluded) atomicOr(&st->excluded, 1u);
     }
@@ -347,7 +342,9 @@ constexpr int64_t kAggRows = 16384;
 bool agglomerate_device(const Mat &A, int64_t bmax, double weight, bool additive, bool drop_stalled, Aggregates &out) {
     Context &ctx = *A.ctx;
     const int64_t n = A.nrows;
-    if (n < kAggRows || bmax < 1) return false;
+    // longer rows would not fit the registers, and their ranks take time that is quadratic in their length (an arrow of
+    // 200,000 rows: 75 ms before it was refused)
+    if (n < kAggRows || bmax < 1 || A.max_row > 64) return false;
     const int32_t *rp = A.rowptr.as<int32_t>(), *ci = A.colidx.as<int32_t>();
     const double *v = A.vals.as<double>();
     Buffer a_max, word, rank, state;
@@ -368,9 +365,9 @@ bool agglomerate_device(const Mat &A, int64_t bmax, double weight, bool additive
         UGPU_CUDA(cudaStreamSynchronize(ctx.stream));
     };
     read_state();
-    if (h.unfit || h.max_row > 64) return false;
-    auto *kernel = h.max_row <= 8 ? k_agglomerate<1, 8> : h.max_row <= 32 ? k_agglomerate<4, 8> : k_agglomerate<8, 8>;
-    const int lanes = h.max_row <= 8 ? 1 : h.max_row <= 32 ? 4 : 8;
+    if (h.unfit) return false;
+    auto *kernel = A.max_row <= 8 ? k_agglomerate<1, 8> : A.max_row <= 32 ? k_agglomerate<4, 8> : k_agglomerate<8, 8>;
+    const int lanes = A.max_row <= 8 ? 1 : A.max_row <= 32 ? 4 : 8;
     int per_sm = 1;
     UGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0));
     const int grid = int(std::max<int64_t>(
