@@ -496,7 +496,7 @@ private:
         const int g = reduce_grid(n);
         const bool f32 = mode_ == CG_GENERIC && pc_->pc_dtype() == UGPU_F32;
         // K0: p = z + beta p   (plain CG: p = r + beta p)
-        // the solver's own vectors are cudaMalloc'd; only x may be caller memory
+        // the solver's own vectors are whole allocations; only x may be caller memory
         const int vec = al16(x) ? 1 : 0;
         // K0 reduces nothing, so it is not tied to the reductions' fixed grid: full occupancy
         const int gp = int(std::max<int64_t>(1, std::min<int64_t>((n / 2 + kBlock - 1) / kBlock,

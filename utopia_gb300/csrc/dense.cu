@@ -72,7 +72,7 @@ __global__ void k_densify(const int32_t *rp, const int32_t *ci, const V *cv, int
 //   3. the rows below take the rank-8 update; warp 0 updates only the next pivot block and goes on to its
 //      elimination, a chain of dependent operations, while the other warps update the rest.
 // One CTA; bound by the FP64 pipe of one SM (87 k FMAs at two per clock, about 21 us) and what is left of the
-// chain: 59 us (65 with the other warps spread over all four schedulers).  Eliminating column by column with all
+// chain: 55 to 59 us (6 us more with the other warps spread over all four schedulers).  Eliminating column by column with all
 // warps queued the chain's operations behind the updates in that pipe (80-90 us); separate factorisation and
 // inversion kernels took 93 and 145 us.
 constexpr int PB = 8;

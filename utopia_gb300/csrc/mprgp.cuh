@@ -22,8 +22,10 @@ struct QpDev {
 // device does not hold the kernel's CTAs at once, x is as it was.
 struct MprgpResident {
     static bool fits(const Context &c, const Mat &A);
-    // Whether run() makes the power-method estimate itself (lambda = 0): up to two rows per thread.  On larger
-    // problems its 0.6 ms of host round trips is nothing beside the solve.
+    // Whether run() makes the power-method estimate itself (lambda = 0): up to two rows per thread (20 iterations on
+    // 380^2 0.58 ms, on 400^2 with the host's estimate 1.54).  Above, it would save 0.9 ms too, but its sums
+    // round in another order than the separate kernels', and over the thousands of iterations of a large free
+    // boundary the last bits of lambda move the iteration count by a few percent.
     static bool own_power_method(const Context &c, const Mat &A);
     static size_t sum_bytes(const Context &c);
     static bool run(Context &c, const Mat &A, const double *b, double *x, const double *lb, const double *ub, double *fi,

@@ -5,14 +5,14 @@
 // conjugate gradient (cg_resident.cu) every thread owns one to four rows for the whole solve, the rows'
 // vectors (and matrix rows of at most eight entries) stay in registers, and an iteration is two exchanges
 // (gridsync.cuh): (s, A s), (s, g) and the step bound after the product, then the four dots of the step.  An
-// expansion step takes two more: its projected iterate must be complete before g = A x - b, and the dots
+// expansion step takes a third: its projected iterate must be complete before g = A x - b, and the dots
 // follow.  An entry whose column belongs to another CTA forms that row's p = fi - beta_sc p_old itself.
 //
 // The convergence test (a root and a division) of an iteration runs beside the next iteration's first exchange,
 // before which neither x nor g changes.
 // Measured per iteration (four of five are expansion steps), obstacle problems of n = 1024 / 4096 / 16,384 / 65,536 /
-// 90,000 / 160,000 / 302,500: 8.7 / 9.3 / 11.2 / 14.5 / 16.3 / 24.9 / 30.0 us, in separate kernels 44 / 40 / 39 / 40 /
-// 42 / 47 / 59 us (power method included).  Bound by the exchanges (about 2.3 us each, 0.7 us in a cluster), the
+// 90,000 / 160,000 / 302,500: 8.8 / 9.2 / 11.3 / 14.7 / 16.7 / 24.8 / 29.8 us, in separate kernels 42 / 38 / 39 / 41 /
+// 42 / 48 / 58 us (power method included).  Bound by the exchanges (about 2.3 us each, 0.7 us in a cluster), the
 // chain of dependent FP64 operations (60 cycles each) around them, and the FP64 pipe on large problems.
 // The step bound divides exactly only where a row's single-precision bracket reaches below the least upper
 // end of the CTA's brackets; the minimum is the one all rows' exact quotients give.
@@ -547,6 +547,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_mprgp_resident(MprgpArgs a) {
 
 }  // namespace
 
+// Rows of at most eight entries: up to four rows per thread (311,296 rows; the times are above).  Longer ones, up to
+// two rows per thread and 32 entries: random graphs of 2001 / 60,001 / 100,001 / 150,001 rows 18 / 22 / 33 / 37 us per
+// iteration against 33 / 42 / 46 / 49 in separate kernels, but 73 against 57 at 200,001.
 bool MprgpResident::fits(const Context &c, const Mat &A) {
     if (A.nrows < 1 || A.max_row <= 0) return false;
     const int64_t threads = int64_t(c.sms) * kThreads;

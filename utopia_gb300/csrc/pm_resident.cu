@@ -185,7 +185,8 @@ __global__ void __launch_bounds__(32) k_lonely_exchange(char *sums, long long li
 
 }  // namespace
 
-// Up to two rows per thread (155,648 rows) of at most 32 entries
+// Up to two rows per thread (155,648 rows) of at most 32 entries: random graphs of 2001 / 20,001 / 60,001 / 150,001 rows
+// 6 / 7 / 10 / 34 us per iteration against 21 / 24 / 25 / 35 in separate kernels, 27 points 64,000 rows 13 / 28.
 bool pm_resident_fits(const Context &c, const Mat &A) {
     return A.nrows >= 1 && A.max_row > 0 && A.max_row <= 32 && A.nrows <= int64_t(c.sms) * kThreads * 2;
 }

@@ -785,7 +785,7 @@ __global__ void UGPU_SELL_BOUNDS k_sell_spmv(SellView m, EpiParams<T> e) {
 // flight together, half as many rows per warp need half as many gathers, and twice as many warps run: a level of
 // 32,768 rows with 27 points took 15 to 17 us in a V-cycle, a V-cycle CG iteration on 128^3 0.78 ms and takes 0.72.
 // A row's products add in the same order as above: the same bits.
-constexpr int kRowSlots = 9;  // a 27-point row in three rounds, a 7- or 9-point row in one
+constexpr int kRowSlots = 9;  // a 27-point row in three rounds (rows of nine entries and fewer stay with the kernel above)
 template <int EPI>
 __global__ void __launch_bounds__(kSpmvWarps * 32, 3) k_sell_rows(SellView m, EpiParams<double> e) {
     if ((e.done && *e.done) || (e.gate && !*e.gate)) return;
